@@ -177,6 +177,10 @@ __global__ void __launch_bounds__(THREADS, pass_min_blocks<THREADS, sizeof(T)>()
           if (ps == 0) batch_contig<T, THREADS, OP_FWD>(I, bt.tile, smraw);
           else if (ps == 2) batch_contig<T, THREADS, OP_INV, OP_POT, OP_FWD>(I, bt.tile, smraw);
           else batch_contig<T, THREADS, OP_INV>(I, bt.tile, smraw);
+          // the lines of a contiguous tile only synchronise among themselves,
+          // and the next tile may lay the shared buffer out for another line
+          // length: no warp may enter it while another still exchanges
+          __syncthreads();
         }
       } else {
         for (int k = blockIdx.x; k < d.nst; k += gridDim.x) {

@@ -63,6 +63,18 @@ def test_batch_matches_single(b200, time):
         assert rel(g, w) <= 1e-15
 
 
+@pytest.mark.parametrize("prec", [0, capi.GRID_PREC_FP32])
+def test_batch_many_mixed_sizes(b200, prec):
+    """Sizes in turn and far more tiles than resident CTAs, so that every CTA
+    of the persistent plans walks from one line length to another many times
+    (all plans run: the first eight steps time them)."""
+    inst = _instances([(1, n, n) for n in (64, 128, 256, 512)] * 16, 17)
+    got, _ = _run(b200, inst, 0.05, 9, True, prec=prec)
+    want, _ = _run(b200, inst, 0.05, 9, False, prec=prec)
+    for i, (g, w) in enumerate(zip(got, want)):
+        assert rel(g, w) <= (1e-7 if prec else 1e-15), i
+
+
 def test_batch_fp32_matches_single(b200):
     inst = _instances(SHAPES[:4], 5)
     got, _ = _run(b200, inst, 0.05, 10, True, prec=capi.GRID_PREC_FP32)
