@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
   } else {
     o = blockIdx.y;
     col0 = (long) blockIdx.x * lpc;
-    nl = lpc;
+    const long rem = a.inner - col0;
+    nl = (int) (rem < lpc ? rem : lpc);
   }
   const double2 zero = make_double2(0.0, 0.0);
 
@@ -923,9 +924,9 @@ static void build_fast_tables(long n, int bc, cd cp, cd c2, int nseg, FastTables
   t.inv_den = make_double2(id.real(), id.imag());
 }
 
-static long largest_pow2_divisor(long v, long cap) {
+static long pow2_at_most(long v) {
   long p = 1;
-  while (p < cap && v % (p * 2) == 0) p *= 2;
+  while (p * 2 <= v) p *= 2;
   return p;
 }
 
@@ -1195,13 +1196,16 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         long cap = (long) (budget / (a.n * 16));
         if (cap > 32) cap = 32;
         if (cap < 1) return gb__set_error(1011, "cn: line too long for a shared-memory tile");
-        const long lpc = largest_pow2_divisor(a.inner, cap);
+        // tiles of 32 columns (or the largest power of two that fits), the
+        // last one partial: a tile as wide as the common power of two of the
+        // extents would be a single column on odd grids
+        const long lpc = pow2_at_most(cap);
         a.lpc = (int) lpc;
         const size_t sm = (size_t) lpc * a.n * 16;
         const FastKernel kern = fast_kernel<false>(a.n);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         if (a.outer > 65535) return gb__set_error(1012, "cn: outer extent above 65535");
-        dim3 grid((unsigned) (a.inner / lpc), (unsigned) a.outer);
+        dim3 grid((unsigned) ((a.inner + lpc - 1) / lpc), (unsigned) a.outer);
         {
           const int slot = gb__pass_begin(15 + axis);
           kern<<<grid, 32 * kSeg, sm, st>>>((double2 *) psi, a);

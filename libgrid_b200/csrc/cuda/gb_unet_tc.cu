@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
   unsigned char *b_sm = smraw + (size_t) p.c8 * plane_bytes;
   // A descriptor of MMA j for the first M-tile (m0 = sz): K-chunks 2j and
   // 2j + 1 (tap, channel chunk), their distance as the leading-byte offset
-  __shared__ uint64_t s_ad[kTcMaxMma];
+  __shared__ uint64_t s_ad[kTcMaxMma + 1];  // one past the last MMA is read ahead, never used
   {
     const uint32_t ab = smem_u32(a_sm);
     const int nkc = 27 * p.c8;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(&bar, 1);
+    mbar_init(&bar, kTcThreads / 32);  // one commit per issuing warp
     fence_mbar_init();
   }
   // B operand (this channel chunk's packed weights) into shared memory
@@ -240,19 +240,31 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
 
   for (int b0 = 0, batch = 0; b0 < p.ntile; b0 += p.tb, batch++) {
     const int nt = min(p.tb, p.ntile - b0);
-    if (tid == 0) {
-      // tile k of the batch starts (b0 + k) * kTcM positions (16-byte units)
-      // after the first tile: added to the start-address field of the
-      // tabled A descriptors (the sum stays inside shared memory, below the
-      // field's 14-bit range); B of MMA j starts j * 2 * np units after B's
+    // Lane 0 of warp k issues the MMAs of the batch's tiles k, k + 8, ...: the
+    // issue of one MMA is a chain of a descriptor read, an add and the move of
+    // its operands to uniform registers, several times longer than the MMA
+    // itself, so one issuing thread left the tensor pipe idle most of the
+    // time.  Tile t starts (b0 + t) * kTcM positions (16-byte units) after the
+    // first tile: added to the start-address field of the tabled A descriptors
+    // (the sum stays inside shared memory, below the field's 14-bit range); B
+    // of MMA j starts j * 2 * np units after B's.
+    if (lane == 0) {
       const uint64_t bd0 = smem_desc(b_base, 16u * (uint32_t) p.np, 128u);
-      for (int k = 0; k < nt; k++) {
+      for (int k = warp; k < nt; k += kTcThreads / 32) {
         const uint64_t moff = (uint64_t) ((b0 + k) * kTcM);
-        for (int j = 0; j < p.nmma; j++)
-          tc_mma(tmem + (uint32_t) (k * p.np), s_ad[j] + moff, bd0 + (uint64_t) (j * 2 * p.np), idesc, j > 0 ? 1u : 0u);
+        const uint32_t dt = tmem + (uint32_t) (k * p.np);
+        uint64_t an = s_ad[0] + moff, bd = bd0;
+#pragma unroll 4
+        for (int j = 0; j < p.nmma; j++) {
+          const uint64_t ac = an;
+          an = s_ad[j + 1] + moff;
+          tc_mma(dt, ac, bd, idesc, j > 0 ? 1u : 0u);
+          bd += (uint64_t) (2 * p.np);
+        }
       }
       tc_commit(&bar);
     }
+    __syncwarp();
     if (!mbar_wait_bounded(&bar, (unsigned) (batch & 1))) ok = false;
     if (__syncthreads_or(!ok)) break;
     tc_fence_after();
@@ -655,9 +667,9 @@ bool tc_plan(int cx, int ny, int d, int h, int w, TcPlan &pl) {
     pl.ntile = (tz * sz + kTcM - 1) / kTcM;
     pl.tb = std::max(1, std::min(pl.ntile, 128 / pl.np));
     pl.ncols = pow2_at_least(pl.tb * pl.np);
-    // at least 57 KB of shared memory per CTA: at most four CTAs (4 x 128
+    // at least 52 KB of shared memory per CTA: at most four CTAs (4 x 128
     // TMEM columns) share an SM
-    pl.smem = std::max(smem, (size_t) 57 * 1024);
+    pl.smem = std::max(smem, (size_t) 52 * 1024);
     return true;
   }
   return false;

@@ -133,6 +133,39 @@ def test_batched_weight_gradient_vs_oracle(lib, engine, cin, cout, shape):
     d.free()
 
 
+@pytest.mark.parametrize("half,off", [((1, 1, 1), 0), ((2, 3, 3), 0), ((3, 1, 6), 0), ((2, 2, 4), 1), ((2, 5, 300), 0)])
+def test_pool_up_relu_shapes(lib, half, off):
+    """Vector and scalar forms of pooling, upsampling and the ReLU mask: odd
+    rows and arrays that start off a 16-byte boundary (off floats) take the
+    scalar one.  Means and sums of eight FP32 values in the oracle's order to
+    8 roundings (1e-6); copies and masks exactly."""
+    rng = np.random.default_rng(5)
+    d, c = Dev(lib), 3
+    full = tuple(2 * s for s in half)
+
+    def put(a):
+        return d.put(np.concatenate([np.zeros(off, np.float32), a.ravel()])) + 4 * off
+
+    x, gc = (rng.standard_normal((c,) + s).astype(np.float32) for s in (full, half))
+    dx, dc, dout = put(x), put(gc), put(np.zeros((c,) + half, np.float32))
+    assert lib.gb_unet_pool2_fwd(dx, dout, c, *full) == 0
+    assert _rel(d.get(dout, (c,) + half), uo.pool2_fwd(x)) < 1e-6
+    assert lib.gb_unet_up2_bwd(dx, dout, c, *half) == 0
+    assert _rel(d.get(dout, (c,) + half), uo.up2_bwd(x)) < 1e-6
+    assert lib.gb_unet_pool2_bwd(dc, dx, c, *full) == 0  # accumulates
+    assert _rel(d.get(dx, (c,) + full), x + uo.pool2_bwd(gc)) < 1e-6
+    assert lib.gb_unet_up2_fwd(dc, dx, c, *half) == 0
+    assert np.array_equal(d.get(dx, (c,) + full), uo.up2_fwd(gc).astype(np.float32))
+    n = x.size - 1  # not a multiple of four
+    y, g = rng.standard_normal((2, x.size)).astype(np.float32)
+    y[0] = np.nan
+    dy, dg = put(y), put(g)
+    for m in (n, x.size):
+        assert lib.gb_unet_relu_bwd(dg, dy, m) == 0
+        assert np.array_equal(d.get(dg, m), np.where(y[:m] > 0, g[:m], 0).astype(np.float32))
+    d.free()
+
+
 def test_pool_up_relu_adam_vs_oracle(lib):
     rng = np.random.default_rng(3)
     d = Dev(lib)
