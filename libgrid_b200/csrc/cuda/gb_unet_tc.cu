@@ -6,22 +6,19 @@
 // input channels.  It is run without an im2col matrix: a CTA stages a
 // zero-padded halo block of the input in shared memory as bf16 channel-chunk
 // planes [c8][position][8 channels] (16 bytes per position), and the A
-// operand of tap t is the same plane read from a start address shifted by
-// off(t) positions.  In the layout tcgen05.mma calls K-major without swizzle,
-// eight consecutive positions form one 8 x 16-byte core matrix, so the shift
-// needs no data movement.  Two K-chunks of 8 channels (two taps, or two
-// channel chunks) make one K = 16 instruction; their distance is the
+// operand of a tap is the same plane read from a start address shifted by the
+// tap's offset in positions.  In the layout tcgen05.mma calls K-major without
+// swizzle, eight consecutive positions form one 8 x 16-byte core matrix, so
+// the shift needs no data movement.  Two K-chunks of 8 channels (two taps, or
+// two channel chunks) make one K = 16 instruction; their distance is the
 // descriptor's leading-byte offset.  M-tiles of 128 consecutive staged
-// positions also cover the halo rows and pad columns; those rows compute
-// values that are never stored, which costs tensor-core time the memory-bound
-// layers have to spare.  The accumulators live in tensor memory (TMEM,
-// 128 columns per CTA), are read back with tcgen05.ld by four warps (one per
-// 32-lane quarter), and the epilogue adds the bias, applies the ReLU and
-// stores FP32 outputs of the interior positions.  A CTA computes 16 output
-// channels (N = 16); wider layers use one CTA per 16 channels of a block, so
-// the weight operand of a CTA (27 taps x input channels x 16) always fits
-// shared memory.  One thread issues the MMAs and commits them to an
-// mbarrier; every wait is bounded.
+// positions cover the pad columns too; those rows compute values that are
+// never stored.  The accumulators live in tensor memory (TMEM), are
+// read back with tcgen05.ld by four warps (one per 32-lane quarter), and the
+// epilogue adds the bias, applies the ReLU and stores FP32 outputs.  A CTA
+// computes 16 output channels; wider layers use one CTA per 16 channels
+// of a block.  CTAs are persistent and lay the weights out in shared memory
+// once.  Every wait is bounded.
 //
 // Weight gradient (mma.sync m16n8k16 bf16, FP32 accumulate):
 //   gw[co][ci][t] += sum_q gy[co][q] x[ci][q + off(t)].
@@ -46,6 +43,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "gb_common.cuh"
 #include "gb_internal_cuda.h"
@@ -115,65 +113,79 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 
 // ---------------------------------------------------------- forward (tcgen05)
 
-constexpr int kTcThreads = 256;  // two warpgroups: staging, epilogue
+constexpr int kTcThreads = 256;  // eight warps: staging, MMA issue (lane 0 of each), epilogue
 constexpr int kTcM = 128;
-constexpr int kTcN = 16;  // output channels per CTA
-constexpr int kStageG = 4;  // staging items whose loads are issued together
-constexpr int kTcMaxMma = 256;  // MMAs per M-tile (K = 27 taps x channels / 16)
+constexpr int kTcN = 16;         // output channels per CTA
+constexpr int kStageU = 4;       // staging items (8 channels of a position) a thread loads before any store
+constexpr int kTcMaxMma = 256;   // MMAs per M-tile (27 taps x channel chunks / 2)
 
-struct TcConv {
-  const float *x;     // [cx][d][h][w] FP32
-  float *y;           // [ny][d][h][w] FP32
-  const float *bias;  // [ny] or null
-  const uint4 *bp;    // packed B: per 16-channel chunk, nmma * 4 core matrices
-  int *err;
-  int cx, ny;         // input channels (K side), output channels (N side)
-  int d, h, w;        // d: all samples' planes (nb x dp)
-  int dp;             // planes per sample (depth neighbours never cross samples)
-  int relu;
-  int tz, ty;         // output block: tz x ty x w voxels
-  int c8, np, nmma;   // channel chunks, N per CTA (16), MMAs per M-tile
-  int sy, sz;         // staged strides (positions)
-  int guard;          // rows before position 0 of a plane
-  int plane_rows;
-  int ntile, tb;      // M-tiles per CTA, M-tiles per TMEM batch
-  int ncols;          // allocated TMEM columns
+// Quotients by a divisor fixed at launch: i / d = umulhi(i, ceil(2^32 / d)),
+// exact while i d < 2^32 (here i and d are staged positions, below 2^15).
+struct FastDiv {
+  uint32_t d, m;
+  __device__ __forceinline__ uint32_t div(uint32_t i) const { return __umulhi(i, m); }
 };
 
-// tap t = 9 (dz + 1) + 3 (dy + 1) + (dx + 1): offset in staged positions
-__device__ __forceinline__ int tap_off(int t, int sy, int sz) {
-  return (t / 9 - 1) * sz + ((t / 3) % 3 - 1) * sy + (t % 3 - 1);
-}
+struct TcConv {
+  const float *x;             // [cx][d][h][w] FP32
+  float *y;                   // [ny][d][h][w] FP32
+  const float *bias;          // [ny] or null
+  const __nv_bfloat16 *wt;    // [cout][cin][27]
+  int *err;
+  int cin, cout;              // of the layer
+  int cx, ny;                 // input channels (K side), output channels (N side)
+  int d, h, w;                // d: all samples' planes (nb x dp)
+  int dp;                     // planes per sample (depth neighbours never cross samples)
+  int relu, mode;             // mode 0: forward, 1: data gradient
+  int wvec;                   // weights read eight at a time
+  int tz, ty, tx;             // output block: tz x ty x tx voxels
+  int nbx, nby, nblk;         // blocks along x and y, blocks in all
+  int c8;                     // channel chunks of 8
+  FastDiv sy, sz, npos;       // staged strides and positions per channel chunk
+  int plane_rows;             // 16-byte rows per channel chunk (guard rows included)
+  int ntm, ntile, tb;         // M-tiles per plane, per block, per TMEM batch
+  int nmma;                   // MMAs per M-tile
+  int ncols;                  // allocated TMEM columns
+};
 
-__global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
+// One CTA walks over its output blocks (tz x ty x tx voxels, 16 output
+// channels).  Block by block it stages the halo block as bf16, runs the MMAs
+// and stores the results; two to three CTAs per SM overlap each other's
+// phases.  (8 -> 8 channels at 128^3: 203 -> 89 us, 24 -> 8: 969 -> 302 us
+// against one CTA per block of whole rows, whose staging took five 32-bit
+// divisions per item and whose weights came from a packing kernel before
+// every launch; 134 and 268 MB of activations, 20 and 41 us of HBM time.
+// What is left is 14 resp. 41 MMAs of about 34 cycles per M-tile, bound by
+// the read of the A operand from shared memory (tensor work 25 / 75 us), and
+// phases that two or three CTAs overlap only in part.)  The K-chunks of an output are added in the order channel chunk,
+// tap (two per MMA), whatever the block shape, so every shape gives the same
+// bits.
+__global__ void __launch_bounds__(kTcThreads, 3) k_conv3_tc(TcConv p) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tslot;
+  __shared__ float s_bias[kTcN];
+  __shared__ uint64_t s_ad[kTcMaxMma + 1];  // one past the last MMA is read ahead, never used
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nby = p.h / p.ty;
-  const int z0 = (blockIdx.x / nby) * p.tz, y0 = (blockIdx.x % nby) * p.ty;
   const int n0 = blockIdx.y * kTcN;  // first output channel of this CTA
-  const int zlo = (z0 / p.dp) * p.dp;  // first plane of this block's sample
   const long vol = (long) p.d * p.h * p.w;
   const uint32_t plane_bytes = (uint32_t) p.plane_rows * 16u;
   unsigned char *a_sm = smraw;
-  unsigned char *b_sm = smraw + (size_t) p.c8 * plane_bytes;
-  // A descriptor of MMA j for the first M-tile (m0 = sz): K-chunks 2j and
-  // 2j + 1 (tap, channel chunk), their distance as the leading-byte offset
-  __shared__ uint64_t s_ad[kTcMaxMma + 1];  // one past the last MMA is read ahead, never used
-  {
+  __nv_bfloat16 *b_sm = (__nv_bfloat16 *) (smraw + (size_t) p.c8 * plane_bytes);
+  const int nkc = 27 * p.c8;  // K-chunks: (channel chunk, tap)
+  // A descriptors of MMA i (K-chunks 2i, 2i + 1) for the first plane and
+  // M-tile: plane dz, row dy, column dx - 1; an odd last chunk is paired with
+  // itself and zero weights
+  for (int i = tid; i < p.nmma; i += kTcThreads) {
     const uint32_t ab = smem_u32(a_sm);
-    const int nkc = 27 * p.c8;
-    for (int j = threadIdx.x; j < p.nmma; j += kTcThreads) {
-      const int k1 = 2 * j, k2 = (2 * j + 1 < nkc) ? 2 * j + 1 : 2 * j;
-      const uint32_t a1 =
-          ab + (uint32_t) (k1 / 27) * plane_bytes + (uint32_t) (p.guard + p.sz + tap_off(k1 % 27, p.sy, p.sz)) * 16u;
-      const uint32_t a2 =
-          ab + (uint32_t) (k2 / 27) * plane_bytes + (uint32_t) (p.guard + p.sz + tap_off(k2 % 27, p.sy, p.sz)) * 16u;
-      s_ad[j] = smem_desc(a1, a2 - a1, 128u);
-    }
+    auto at = [&](int kc) {
+      const int c = kc / 27, t = kc - c * 27;
+      return ab + (uint32_t) c * plane_bytes +
+             (1u + (uint32_t) (t / 9) * p.sz.d + (uint32_t) (t / 3 % 3) * p.sy.d + (uint32_t) (t % 3) - 1u) * 16u;
+    };
+    const uint32_t a1 = at(2 * i), a2 = at(2 * i + 1 < nkc ? 2 * i + 1 : 2 * i);
+    s_ad[i] = smem_desc(a1, a2 - a1, 128u);
   }
-
   if (warp == 0) {
     tmem_alloc(&tslot, (uint32_t) p.ncols);
     tmem_relinquish();
@@ -182,119 +194,168 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
     mbar_init(&bar, kTcThreads / 32);  // one commit per issuing warp
     fence_mbar_init();
   }
-  // B operand (this channel chunk's packed weights) into shared memory
-  const int nb16 = p.nmma * 2 * (kTcN / 8) * 8;  // 16-byte units
-  const uint4 *bsrc = p.bp + (size_t) blockIdx.y * nb16;
-  for (int i = tid; i < nb16; i += kTcThreads) ((uint4 *) b_sm)[i] = bsrc[i];
-  // A operand: the zero-padded halo block, bf16 channel-chunk planes.  The
-  // work items are (staged row, 32-position chunk of the row), lanes along
-  // x; a warp takes every 8th item and issues the loads of kStageG items
-  // (8 channels each) before packing and storing any of them, so that many
-  // loads are in flight per lane instead of one row chunk at a time.
+  // weights: zeros (channels past the layer's, the odd chunk's partner), then
+  // the layer's, read in memory order
+  for (int i = tid; i < p.nmma * 2 * kTcN; i += kTcThreads) ((uint4 *) b_sm)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
   {
-    constexpr int G = kStageG, NW = kTcThreads / 32;
-    const int rows_per_plane = (p.tz + 2) * (p.ty + 2);
-    const int xch = (p.sy + 31) >> 5;
-    const int nitems = p.c8 * rows_per_plane * xch;
-    for (int i0 = warp; i0 < nitems; i0 += G * NW) {
-      float v[G][8];
-      int dpos[G];
+    // runs of consecutive weights: the whole chunk [n][c][t] (forward), or
+    // per channel c the run [n][26 - t] (data gradient)
+    const int nn = min(kTcN, p.ny - n0);
+    const int runlen = p.mode == 0 ? nn * p.cx * 27 : nn * 27, nruns = p.mode == 0 ? 1 : p.cx;
+    const size_t first = (size_t) n0 * 27 * (p.mode == 0 ? p.cx : 1), pitch = (size_t) p.cin * 27;
+    const unsigned short *wp = (const unsigned short *) p.wt + first;
+    // element r of run c0 -> (n, c, t) and on to the next
+    auto put = [&](int n, int c, int t, unsigned short v) {
+      ((unsigned short *) b_sm)[(((c >> 3) * 27 + t) * kTcN + n) * 8 + (c & 7)] = v;
+    };
+    if (p.wvec) {  // eight weights per load
+      const int per = runlen / 8;
+#pragma unroll 4
+      for (int i = tid; i < per * nruns; i += kTcThreads) {
+        const int run = i / per, r = (i - run * per) * 8;
+        const uint4 q = __ldg((const uint4 *) (wp + (size_t) run * pitch) + (i - run * per));
+        const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+        int n, c = run, t = r % 27;
+        if (p.mode == 0) {
+          n = r / (27 * p.cx);
+          c = r / 27 - n * p.cx;
+        } else {
+          n = r / 27;
+        }
 #pragma unroll
-      for (int g = 0; g < G; g++) {
-        const int it = i0 + g * NW;
-        dpos[g] = -1;
-#pragma unroll
-        for (int e = 0; e < 8; e++) v[g][e] = 0.f;
-        if (it < nitems) {
-          const int row = it / xch, xc = it - row * xch;
-          const int c = row / rows_per_plane, rr = row - c * rows_per_plane;
-          const int zs = rr / (p.ty + 2), ys = rr - zs * (p.ty + 2);
-          const int xs = xc * 32 + lane;
-          if (xs < p.sy) {
-            dpos[g] = c * p.plane_rows + p.guard + zs * p.sz + ys * p.sy + xs;
-            const int z = z0 + zs - 1, y = y0 + ys - 1, x = xs - 1;
-            if (z >= zlo && z < zlo + p.dp && y >= 0 && y < p.h && x >= 0 && x < p.w) {
-              const float *src = p.x + ((long) z * p.h + y) * p.w + x;
-#pragma unroll
-              for (int e = 0; e < 8; e++)
-                if (c * 8 + e < p.cx) v[g][e] = __ldg(src + (size_t) (c * 8 + e) * vol);
-            }
+        for (int e = 0; e < 8; e++) {
+          put(n, c, p.mode == 0 ? t : 26 - t, (unsigned short) (u[e >> 1] >> (16 * (e & 1))));
+          if (++t == 27) {
+            t = 0;
+            if (p.mode != 0) n++;
+            else if (++c == p.cx) c = 0, n++;
           }
         }
       }
-#pragma unroll
-      for (int g = 0; g < G; g++)
-        if (dpos[g] >= 0)
-          ((uint4 *) a_sm)[dpos[g]] = make_uint4(pack_bf16x2(v[g][0], v[g][1]), pack_bf16x2(v[g][2], v[g][3]),
-                                                 pack_bf16x2(v[g][4], v[g][5]), pack_bf16x2(v[g][6], v[g][7]));
+    } else {
+      for (int i = tid; i < runlen * nruns; i += kTcThreads) {
+        const int run = i / runlen, r = i - run * runlen, t = r % 27;
+        const unsigned short v = __ldg(wp + (size_t) run * pitch + r);
+        if (p.mode == 0) {
+          const int n = r / (27 * p.cx);
+          put(n, r / 27 - n * p.cx, t, v);
+        } else {
+          put(r / 27, run, 26 - t, v);
+        }
+      }
     }
   }
-  fence_proxy_async_smem();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tslot;
+  if (tid < kTcN) s_bias[tid] = (p.bias && n0 + tid < p.ny) ? __ldg(p.bias + n0 + tid) : 0.f;
   const uint32_t b_base = smem_u32(b_sm);
-  const uint32_t idesc = idesc_bf16(kTcM, p.np);
+  const int nitems = p.c8 * (int) p.npos.d;
   bool ok = true;
+  uint32_t phase = 0;
 
-  for (int b0 = 0, batch = 0; b0 < p.ntile; b0 += p.tb, batch++) {
-    const int nt = min(p.tb, p.ntile - b0);
-    // Lane 0 of warp k issues the MMAs of the batch's tiles k, k + 8, ...: the
-    // issue of one MMA is a chain of a descriptor read, an add and the move of
-    // its operands to uniform registers, several times longer than the MMA
-    // itself, so one issuing thread left the tensor pipe idle most of the
-    // time.  Tile t starts (b0 + t) * kTcM positions (16-byte units) after the
-    // first tile: added to the start-address field of the tabled A descriptors
-    // (the sum stays inside shared memory, below the field's 14-bit range); B
-    // of MMA j starts j * 2 * np units after B's.
-    if (lane == 0) {
-      const uint64_t bd0 = smem_desc(b_base, 16u * (uint32_t) p.np, 128u);
-      for (int k = warp; k < nt; k += kTcThreads / 32) {
-        const uint64_t moff = (uint64_t) ((b0 + k) * kTcM);
-        const uint32_t dt = tmem + (uint32_t) (k * p.np);
-        uint64_t an = s_ad[0] + moff, bd = bd0;
-#pragma unroll 4
-        for (int j = 0; j < p.nmma; j++) {
-          const uint64_t ac = an;
-          an = s_ad[j + 1] + moff;
-          tc_mma(dt, ac, bd, idesc, j > 0 ? 1u : 0u);
-          bd += (uint64_t) (2 * p.np);
-        }
-      }
-      tc_commit(&bar);
-    }
-    __syncwarp();
-    if (!mbar_wait_bounded(&bar, (unsigned) (batch & 1))) ok = false;
-    if (__syncthreads_or(!ok)) break;
-    tc_fence_after();
-    // epilogue: warpgroup g takes tiles k = g, g + 2, ...; warp w reads TMEM
-    // lanes 32 (w % 4) .. + 31 = those rows of a tile
-    const int wq = warp & 3, wg = warp >> 2;
-    for (int k = wg; k < nt; k += kTcThreads / 128) {
-      const int pos = p.sz + (b0 + k) * kTcM + wq * 32 + lane;
-      const int zs = pos / p.sz, rem = pos - zs * p.sz, ys = rem / p.sy, xs = rem - ys * p.sy;
-      const bool useful = zs >= 1 && zs <= p.tz && ys >= 1 && ys <= p.ty && xs >= 1 && xs <= p.w;
-      const long vox = ((long) (z0 + zs - 1) * p.h + (y0 + ys - 1)) * p.w + (xs - 1);
-      for (int nb = 0; nb < p.np; nb += 16) {
-        float v[16];
-        tc_ld16(tmem + ((uint32_t) (wq * 32) << 16) + (uint32_t) (k * p.np + nb), v);
-        if (useful) {
+  for (int blk = blockIdx.x; blk < p.nblk && ok; blk += gridDim.x) {
+    const int br = blk / p.nbx, x0 = (blk - br * p.nbx) * p.tx;
+    const int z0 = (br / p.nby) * p.tz, y0 = (br % p.nby) * p.ty;
+    const int zlo = (z0 / p.dp) * p.dp;  // first plane of this block's sample
+    // A operand: the zero-padded halo block, bf16 channel-chunk planes.  A
+    // thread takes items (channel chunk, position) tid, tid + 256, ... and
+    // issues the loads of kStageU items (8 channels each) before packing and
+    // storing any of them.
+    for (int i0 = tid; i0 < nitems; i0 += kStageU * kTcThreads) {
+      float v[kStageU][8];
+      int dst[kStageU];
 #pragma unroll
-          for (int q = 0; q < 16; q++) {
-            const int co = n0 + nb + q;
-            if (co < p.ny) {
-              float r = v[q] + (p.bias ? __ldg(p.bias + co) : 0.f);
-              if (p.relu) r = fmaxf(r, 0.f);
-              p.y[(size_t) co * vol + vox] = r;
+      for (int u = 0; u < kStageU; u++) {
+        const uint32_t it = (uint32_t) (i0 + u * kTcThreads);
+        dst[u] = -1;
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[u][e] = 0.f;
+        if (it < (uint32_t) nitems) {
+          const uint32_t c = p.npos.div(it), pos = it - c * p.npos.d;
+          const uint32_t zs = p.sz.div(pos), r = pos - zs * p.sz.d, ys = p.sy.div(r), xs = r - ys * p.sy.d;
+          dst[u] = (int) (c * (uint32_t) p.plane_rows + 1u + pos);
+          const int z = z0 + (int) zs - 1, y = y0 + (int) ys - 1, x = x0 + (int) xs - 1;
+          if (z >= zlo && z < zlo + p.dp && (unsigned) y < (unsigned) p.h && (unsigned) x < (unsigned) p.w) {
+            const int cl = (int) c * 8;
+            const float *src = p.x + (size_t) cl * vol + ((long) z * p.h + y) * p.w + x;
+            if (cl + 8 <= p.cx) {
+#pragma unroll
+              for (int e = 0; e < 8; e++) v[u][e] = __ldg(src + (size_t) e * vol);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; e++)
+                if (cl + e < p.cx) v[u][e] = __ldg(src + (size_t) e * vol);
             }
           }
         }
       }
+#pragma unroll
+      for (int u = 0; u < kStageU; u++)
+        if (dst[u] >= 0)
+          ((uint4 *) a_sm)[dst[u]] = make_uint4(pack_bf16x2(v[u][0], v[u][1]), pack_bf16x2(v[u][2], v[u][3]),
+                                                pack_bf16x2(v[u][4], v[u][5]), pack_bf16x2(v[u][6], v[u][7]));
     }
+    fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    const uint32_t tmem = tslot;
+
+    for (int b0 = 0; b0 < p.ntile; b0 += p.tb) {
+      const int nt = min(p.tb, p.ntile - b0);
+      // Lane 0 of warp k issues the MMAs of the batch's tiles k, k + 8, ...: the
+      // issue of one MMA is a chain of a descriptor read, an add and the move
+      // of its operands to uniform registers, longer than the MMA itself.
+      if (lane == 0) {
+        const uint32_t id = idesc_bf16(kTcM, kTcN);
+        for (int k = warp; k < nt; k += kTcThreads / 32) {
+          const int tile = b0 + k, g = tile / p.ntm, m = tile - g * p.ntm;
+          const uint64_t ao = (uint64_t) g * p.sz.d + (uint64_t) (m * kTcM);
+          const uint32_t dt = tmem + (uint32_t) (k * kTcN);
+          uint64_t an = s_ad[0] + ao, bd = smem_desc(b_base, 16u * kTcN, 128u);
+#pragma unroll 4
+          for (int i = 0; i < p.nmma; i++) {
+            const uint64_t ac = an;
+            an = s_ad[i + 1] + ao;
+            tc_mma(dt, ac, bd, id, i > 0 ? 1u : 0u);
+            bd += 2u * kTcN;
+          }
+        }
+        tc_commit(&bar);
+      }
+      __syncwarp();
+      if (!mbar_wait_bounded(&bar, phase)) ok = false;
+      phase ^= 1u;
+      if (__syncthreads_or(!ok)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      // epilogue: warpgroup g takes tiles k = g, g + 2, ...; warp w reads TMEM
+      // lanes 32 (w % 4) .. + 31 = those rows of a tile
+      const int wq = warp & 3, wg = warp >> 2;
+      for (int k = wg; k < nt; k += kTcThreads / 128) {
+        const int tile = b0 + k, g = tile / p.ntm, m = tile - g * p.ntm;
+        const uint32_t r = (uint32_t) (m * kTcM + wq * 32 + lane), ys = p.sy.div(r), xs = r - ys * p.sy.d;
+        const bool useful = (int) ys < p.ty && xs >= 1 && (int) xs <= p.tx;
+        const long hw = (long) p.h * p.w;
+        const long vox = (long) (z0 + g) * hw + (long) (y0 + (int) ys) * p.w + (x0 + (int) xs - 1);
+        float v[16];
+        tc_ld16(tmem + ((uint32_t) (wq * 32) << 16) + (uint32_t) (k * kTcN), v);
+        if (useful) {
+#pragma unroll
+          for (int q = 0; q < kTcN; q++) {
+            if (n0 + q < p.ny) {
+              float o = v[q] + s_bias[q];
+              if (p.relu) o = fmaxf(o, 0.f);
+              p.y[(size_t) (n0 + q) * vol + vox] = o;
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+    }
   }
   if (!ok) {
     // an MMA batch never completed: record it and let it drain (bounded)
@@ -306,38 +367,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc(TcConv p) {
     tc_fence_before();
     __syncthreads();
   }
-  if (warp == 0) tmem_dealloc(tmem, (uint32_t) p.ncols);
-}
-
-// Packed B operand, per chunk of 16 output channels nc: for MMA j and
-// K-chunk h (chunk kc = 2 j + h, tap kc % 27, channel chunk kc / 27), the
-// 16 x 8 block of weights as two core matrices of 8 rows (n) x 8 bf16
-// (channels), [nc][j][h][ng][row][e].  mode 0 (forward): B_t[n][c] =
-// w[n][c][t]; mode 1 (data gradient): B_t[n][c] = w[c][n][26 - t] with n an
-// input channel and c an output channel of the layer.
-__global__ void k_pack_b(const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ bp, int cin, int cout,
-                         int nch, int c8, int nmma, int mode) {
-  const long per = (long) nmma * 2 * kTcN * 8;  // elements per channel chunk
-  const long total = per * nch;
-  const long i = (long) blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int nc = (int) (i / per);
-  const long r0 = i - nc * per;
-  const int e = (int) (r0 % 8), row = (int) ((r0 / 8) % 8);
-  const long rest = r0 / 64;
-  const int ng = (int) (rest % (kTcN / 8));
-  const int kc = (int) (rest / (kTcN / 8));  // 2 j + h
-  const int n = nc * kTcN + ng * 8 + row;
-  __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-  if (kc < 27 * c8) {
-    const int t = kc % 27, c = (kc / 27) * 8 + e;
-    if (mode == 0) {
-      if (n < cout && c < cin) v = w[((size_t) n * cin + c) * 27 + t];
-    } else {
-      if (n < cin && c < cout) v = w[((size_t) c * cin + n) * 27 + (26 - t)];
-    }
-  }
-  bp[i] = v;
+  if (warp == 0) tmem_dealloc(tslot, (uint32_t) p.ncols);
 }
 
 // ------------------------------------------------ weight gradient (mma.sync)
@@ -632,7 +662,7 @@ __global__ void k_wgrad_reduce_t(const float *__restrict__ part, float *__restri
 int g_tc_on = 1;
 
 struct TcPlan {
-  int tz, ty, c8, np, nch, nmma, sy, sz, guard, plane_rows, ntile, tb, ncols;
+  int tz, ty, tx, c8, nch, nmma, plane_rows, npos, ntm, ntile, tb, ncols, ctas;
   size_t smem;
 };
 
@@ -642,86 +672,123 @@ int pow2_at_least(int v) {
   return p;
 }
 
-bool tc_plan(int cx, int ny, int d, int h, int w, TcPlan &pl) {
+int num_sms() {
+  int nsm = 148, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+
+// Block shape: the candidate with the least estimated time.  A CTA alone
+// spends about 46 cycles per warp item of staging, 34 per MMA, 360 per M-tile
+// of the epilogue and 4400 besides; CTAs that share an SM overlap each other's
+// phases down to the time of the tensor pipe.  A last round that is not full
+// costs 0.6 of a round.  Fitted on B200 to the times of 16 layers (3 -> 8
+// channels at 128^3 to 64 -> 64 at 4^3 x 8) in up to 25 block shapes each:
+// 13 layers get a shape within 5% of their fastest, the worst are 24 -> 8 at
+// 128^3 (302 us, best 273) and 64 -> 64 at 16^3 (27 us, best 21).
+bool tc_plan(int cx, int ny, int nb, int d, int h, int w, int nsm, TcPlan &best) {
+  double best_cost = -1.0;
+  TcPlan pl;
   pl.c8 = (cx + 7) / 8;
-  pl.np = kTcN;
   pl.nch = (ny + kTcN - 1) / kTcN;
   pl.nmma = (27 * pl.c8 + 1) / 2;
   if (pl.nmma > kTcMaxMma) return false;
-  const size_t bbytes = (size_t) pl.nmma * 32 * pl.np;
-  const int cand[5][2] = {{4, 4}, {4, 2}, {2, 2}, {2, 1}, {1, 1}};
-  for (auto &c : cand) {
-    const int tz = c[0], ty = c[1];
-    if (tz > d || ty > h || d % tz || h % ty) continue;
-    const int sy = w + 2, sz = (ty + 2) * sy;
-    const int guard = sy + 1;
-    const int plane_rows = ((tz + 2) * sz + 2 * sy + 129 + 1) & ~1;
-    const size_t smem = (size_t) pl.c8 * plane_rows * 16 + bbytes;
-    if (smem > 200 * 1024) continue;
-    pl.tz = tz;
-    pl.ty = ty;
-    pl.sy = sy;
-    pl.sz = sz;
-    pl.guard = guard;
-    pl.plane_rows = plane_rows;
-    pl.ntile = (tz * sz + kTcM - 1) / kTcM;
-    pl.tb = std::max(1, std::min(pl.ntile, 128 / pl.np));
-    pl.ncols = pow2_at_least(pl.tb * pl.np);
-    // at least 52 KB of shared memory per CTA: at most four CTAs (4 x 128
-    // TMEM columns) share an SM
-    pl.smem = std::max(smem, (size_t) 52 * 1024);
-    return true;
-  }
-  return false;
+  for (int tx = w; tx >= 16 || tx == w; tx = tx % 2 ? 0 : tx / 2)
+    for (int s = 0; s < 20; s++) {
+      const int tz = 8 >> (s / 5), ty = 16 >> (s % 5);
+      if (d % tz || h % ty) continue;
+      pl.tx = tx;
+      pl.tz = tz;
+      pl.ty = ty;
+      const int sy = tx + 2, sz = (ty + 2) * sy;
+      pl.npos = (tz + 2) * sz;
+      pl.ntm = (ty * sy + kTcM - 1) / kTcM;
+      pl.ntile = pl.ntm * tz;
+      // one guard row in front (the tap left of position 0); the last M-tile
+      // of a plane runs past its rows by less than 128 positions, and its
+      // taps reach two rows and one position further
+      pl.plane_rows = std::max(1 + pl.npos, (tz + 1) * sz + 2 * sy + pl.ntm * kTcM + 2);
+      const size_t bytes = ((size_t) pl.c8 * pl.plane_rows + (size_t) (2 * pl.nmma) * kTcN) * 16;
+      if (bytes > 200 * 1024 || pl.npos * pl.c8 >= 32768 || pl.ntm * kTcM >= 32768) continue;
+      // static shared memory and the per-CTA reservation: 3 KB
+      pl.ctas = (int) std::min<size_t>(3, 227 * 1024 / (bytes + 3 * 1024));
+      const int cap = pl.ctas == 1 ? 512 : pl.ctas == 2 ? 256 : 128;  // TMEM columns per CTA
+      pl.tb = std::max(1, std::min(pl.ntile, cap / kTcN));
+      pl.ncols = pow2_at_least(pl.tb * kTcN);
+      pl.smem = bytes;
+      const long total = (long) nb * (d / tz) * (h / ty) * (w / tx) * pl.nch;
+      const int share = (int) std::min<long>(pl.ctas, (total + nsm - 1) / nsm);
+      const double mma = 34.0 * pl.ntile * pl.nmma;
+      const double own = 46.0 * pl.c8 * pl.npos / 32.0 + mma + 360.0 * pl.ntile + 4400.0;
+      const double avg = (double) total / ((double) nsm * share);
+      const double rounds = std::max(1.0, avg + 0.6 * (std::ceil(avg) - avg));
+      const double cost = rounds * std::max(own, share * mma);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best = pl;
+      }
+    }
+  return best_cost >= 0;
 }
 
-int run_conv_tc(const float *x, const uint16_t *w, const float *bias, float *y, int cin, int cout, int nb, int d, int h,
-                int wd, int relu, int mode) {
+FastDiv fast_div(int d) { return FastDiv{(uint32_t) d, (uint32_t) (((1ull << 32) + (unsigned) d - 1) / (unsigned) d)}; }
+
+int run_conv_tc(const TcPlan &pl, int nsm, const float *x, const uint16_t *w, const float *bias, float *y, int cin,
+                int cout, int nb, int d, int h, int wd, int relu, int mode) {
   // mode 0: y[cout] = conv(x[cin]); mode 1: y = gx[cin] from x = gy[cout];
   // nb samples of d planes each, stacked along the depth axis
-  const int cx = mode == 0 ? cin : cout, ny = mode == 0 ? cout : cin;
-  TcPlan pl;
-  if (!tc_plan(cx, ny, d, h, wd, pl)) return gb__set_error(1104, "unet tensor-core conv: no block plan fits");
-  const size_t nbp = (size_t) pl.nmma * 2 * kTcN * 8 * pl.nch;  // bf16 elements
-  __nv_bfloat16 *bp = (__nv_bfloat16 *) gb__scratch(GB_SCR_UNETB, nbp * sizeof(__nv_bfloat16));
   int *err = gb__status(GB_STATUS_PASS);
-  if (!bp || !err) return gb_last_error();
-  cudaStream_t st = gb__stream();
-  k_pack_b<<<(unsigned) ((nbp + 255) / 256), 256, 0, st>>>((const __nv_bfloat16 *) w, bp, cin, cout, pl.nch, pl.c8,
-                                                              pl.nmma, mode);
-  GB_CHECK_LAUNCH("unet pack weights");
+  if (!err) return gb_last_error();
   TcConv p;
   p.x = x;
   p.y = y;
   p.bias = bias;
-  p.bp = (const uint4 *) bp;
+  p.wt = (const __nv_bfloat16 *) w;
   p.err = err;
-  p.cx = cx;
-  p.ny = ny;
+  p.cin = cin;
+  p.cout = cout;
+  p.cx = mode == 0 ? cin : cout;
+  p.ny = mode == 0 ? cout : cin;
   p.d = nb * d;
   p.dp = d;
   p.h = h;
   p.w = wd;
   p.relu = relu;
+  p.mode = mode;
   p.tz = pl.tz;
   p.ty = pl.ty;
+  p.tx = pl.tx;
+  p.nbx = wd / pl.tx;
+  p.nby = h / pl.ty;
+  p.nblk = (nb * d / pl.tz) * p.nby * p.nbx;
   p.c8 = pl.c8;
-  p.np = pl.np;
-  p.nmma = pl.nmma;
-  p.sy = pl.sy;
-  p.sz = pl.sz;
-  p.guard = pl.guard;
+  p.sy = fast_div(pl.tx + 2);
+  p.sz = fast_div((pl.ty + 2) * (pl.tx + 2));
+  p.npos = fast_div(pl.npos);
   p.plane_rows = pl.plane_rows;
+  p.ntm = pl.ntm;
   p.ntile = pl.ntile;
   p.tb = pl.tb;
+  p.nmma = pl.nmma;
+  // eight weights per load: every run starts on 16 bytes and is whole vectors
+  // long (all layers of the network but the data gradient of three channels)
+  const int last = p.ny - (pl.nch - 1) * kTcN;  // channels of the last chunk
+  p.wvec = ((size_t) w & 15) == 0 && (mode == 0 ? (long) last * p.cx % 8 == 0
+                                               : cin % 8 == 0 && last % 8 == 0);
   p.ncols = pl.ncols;
-  static size_t attr = 0;
-  if (pl.smem > attr) {
-    cudaFuncSetAttribute(k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (200 * 1024 + 1024));
-    attr = 200 * 1024 + 1024;
+  static bool attr[kMaxDevices] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  bool &set = attr[dev >= 0 && dev < kMaxDevices ? dev : 0];
+  if (!set) {
+    cudaFuncSetAttribute(k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    set = true;
   }
-  const dim3 grid((unsigned) ((nb * d / pl.tz) * (h / pl.ty)), (unsigned) pl.nch);
-  k_conv3_tc<<<grid, kTcThreads, pl.smem, st>>>(p);
+  // one resident wave; a CTA keeps its weights for all of its blocks
+  const int per = std::max(1, pl.ctas * nsm / pl.nch);
+  const dim3 grid((unsigned) std::min(p.nblk, per), (unsigned) pl.nch);
+  k_conv3_tc<<<grid, kTcThreads, pl.smem, gb__stream()>>>(p);
   GB_CHECK_LAUNCH("unet tensor-core conv");
   return 0;
 }
@@ -865,9 +932,10 @@ extern "C" int gb_unet_tensor_cores(int on) {
 int gb__unet_conv_tc(const float *x, const uint16_t *w, const float *b, float *y, int cin, int cout, int nb, int d,
                      int h, int wd, int relu, int mode) {
   if (!g_tc_on) return -1;
+  const int nsm = num_sms();
   TcPlan pl;
-  if (!tc_plan(mode == 0 ? cin : cout, mode == 0 ? cout : cin, d, h, wd, pl)) return -1;
-  return run_conv_tc(x, w, b, y, cin, cout, nb, d, h, wd, relu, mode);
+  if (!tc_plan(mode == 0 ? cin : cout, mode == 0 ? cout : cin, nb, d, h, wd, nsm, pl)) return -1;
+  return run_conv_tc(pl, nsm, x, w, b, y, cin, cout, nb, d, h, wd, relu, mode);
 }
 
 int gb__unet_wgrad_tc(const float *x, const float *gy, float *gw, float *gb, int cin, int cout, int nb, int d, int h,

@@ -133,6 +133,31 @@ def test_batched_weight_gradient_vs_oracle(lib, engine, cin, cout, shape):
     d.free()
 
 
+@pytest.mark.parametrize("cin,cout,shape,off", [(8, 8, (4, 16, 128), 0), (24, 8, (8, 8, 128), 1), (3, 20, (4, 6, 36), 0),
+                                                (16, 33, (2, 4, 48), 3), (3, 8, (96, 64, 128), 0)])
+def test_conv_blocks_and_weight_alignment(lib, cin, cout, shape, off):
+    """Tensor-core convolutions on rows split into several blocks, with more
+    blocks than resident CTAs, output channels past a multiple of 16, and
+    weights off a 16-byte boundary (off values): operands rounded to bf16,
+    FP32 sums of at most 27 x 33 products (1e-5)."""
+    rng = np.random.default_rng(cout)
+    d = Dev(lib)
+    x = rng.standard_normal((cin,) + shape).astype(np.float32)
+    gy = rng.standard_normal((cout,) + shape).astype(np.float32)
+    w = rng.standard_normal((cout, cin, 27)).astype(np.float32)
+    b = rng.standard_normal(cout).astype(np.float32)
+    dw = d.put(np.concatenate([np.zeros(off, np.uint16), uo.bf16_bits(w).ravel()])) + 2 * off
+    wr = uo.bf16_round(w)
+    dy = d.put(np.zeros((cout,) + shape, np.float32))
+    assert lib.gb_unet_conv3_fwd(d.put(x), dw, d.put(b), dy, cin, cout, *shape, 1) == 0
+    assert _rel(d.get(dy, (cout,) + shape), uo.conv3_fwd(x, wr, b, 1, True)) < TOL_TC
+    if np.prod(shape) < 1e5:
+        dgx = d.put(np.full((cin,) + shape, 7.0, np.float32))
+        assert lib.gb_unet_conv3_bwd_data(d.put(gy), dw, dgx, cin, cout, *shape) == 0
+        assert _rel(d.get(dgx, (cin,) + shape), uo.conv3_bwd_data(gy, wr, True)) < TOL_TC
+    d.free()
+
+
 @pytest.mark.parametrize("half,off", [((1, 1, 1), 0), ((2, 3, 3), 0), ((3, 1, 6), 0), ((2, 2, 4), 1), ((2, 5, 300), 0)])
 def test_pool_up_relu_shapes(lib, half, off):
     """Vector and scalar forms of pooling, upsampling and the ReLU mask: odd
