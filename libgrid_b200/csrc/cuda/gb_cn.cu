@@ -188,7 +188,7 @@ __device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int 
 }
 
 // Potential factor over a whole tile in shared memory.  Contiguous tiles
-// (lines along z, element (l, i) at sm[l * pitch + i]): one line per warp
+// (lines along the last axis longer than 1, element (l, i) at sm[l * pitch + i]): one line per warp
 // at a time, lanes along the line.  Strided tiles (element (l, i) at
 // sm[i * pitch + l], pitch >= cols): one column per thread, `cols` columns
 // side by side, threads of equal column spaced along the rows.
@@ -200,9 +200,16 @@ __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, in
   if constexpr (CONTIG) {
     for (int l = (int) (threadIdx.x >> 5); l < nl; l += nthr >> 5) {
       const long lid = line0 + l;
-      const long ix = lid / a.ny, iy = lid - ix * a.ny;
-      cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, (ix * a.ny + iy) * vrow, 1, ix, iy, 0,
-                   a, pt);
+      if (a.axis == 2) {
+        const long ix = lid / a.ny, iy = lid - ix * a.ny;
+        cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, (ix * a.ny + iy) * vrow, 1, ix, iy, 0,
+                     a, pt);
+      } else {
+        // without a z axis (nz = 1) the contiguous lines run along y, or along
+        // x when ny = 1 too: their elements lie a potential row apart
+        const long ix = a.axis == 1 ? lid : 0;
+        cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, ix * a.ny * vrow, vrow, ix, 0, 0, a, pt);
+      }
     }
   } else {
     const int l = (int) threadIdx.x % cols;

@@ -228,6 +228,31 @@ def test_cn_step(b200, restate, bc, shape, time):
     assert rel(got, want) < TOL_PSI
 
 
+@pytest.mark.parametrize("bc", [DIR, NEU, PER])
+@pytest.mark.parametrize("shape", [(20, 41, 1), (7, 64, 1), (24, 1, 1), (9, 1, 30)])
+@pytest.mark.parametrize("gp", [False, True])
+def test_cn_step_short_axes(b200, restate, bc, shape, gp):
+    """Grids without a z (and y) axis: the lines of the last sweep are
+    contiguous there, its potential half-step walks over y (x)."""
+    step, mass, g = 0.3, 1.3, 0.02
+    rng = np.random.default_rng(19)
+    psi0 = smooth_state(shape, step) + 0.01 * rand_c(rng, shape)
+    v = 0.05 * rng.standard_normal(shape)
+    for on in (0, 1):  # both line solvers
+        old = b200.lib.gb_cn_warp_solver(on)
+        try:
+            got = b200_cn_run(b200, psi0, None if gp else v, step, mass, 0.05, bc, 3, gp=(v, g) if gp else None)
+        finally:
+            b200.lib.gb_cn_warp_solver(old)
+        want = psi0.copy()
+        for _ in range(3):
+            if gp:
+                want = restate.cn_step(want, step, mass, 0.05, bc, vr=workloads.padded(v), g=g)
+            else:
+                want = restate.cn_step(want, step, mass, 0.05, bc, vc=v.astype(complex))
+        assert rel(got, want) < TOL_PSI
+
+
 @pytest.mark.parametrize("bc", [DIR, PER])
 def test_cn_rotation_and_absorber(b200, restate, bc):
     """General line-solver path: rotating frame and absorbing ramp."""
