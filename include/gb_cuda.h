@@ -188,6 +188,14 @@ int gb_split_step(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_p
  * reference makes one step per call). */
 int gb_split_steps(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_potential *pot, int nsteps);
 
+/* nsteps such steps (imaginary time), each followed by the renormalisation
+ * of gb_normalize_device, with the k-space state kept between them and the
+ * norm taken in k-space: 4 passes per step, no host synchronisation, the same
+ * result to rounding.  Needs a potential and two axes longer than 1.  No
+ * reference counterpart. */
+int gb_relax_steps(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_potential *pot, int nsteps,
+                   double target, double step_factor);
+
 /* k-space multipliers on unshifted frequencies (src/cgrid_diff.c:454-807):
  * dst = src * (-k^2) or src * (i k_axis). */
 #define GB_K_LAPLACE 1

@@ -35,7 +35,11 @@ namespace gbfft {
 // OP_POT_RP is the potential op for one case only, a real V_ext in real
 // time without an absorbing region (a pure phase), so a kernel built for it
 // carries none of the other potential paths.
-enum : int { OP_END = 0, OP_FWD = 1, OP_INV = 2, OP_KIN = 3, OP_POT = 4, OP_SCALE = 5, OP_KSQ = 6, OP_POT_RP = 7 };
+// OP_KIN2 is the kinetic factor twice with the sum of |psi|^2 taken between
+// the two (the end of one step and the start of the next, renormalised).
+enum : int {
+  OP_END = 0, OP_FWD = 1, OP_INV = 2, OP_KIN = 3, OP_POT = 4, OP_SCALE = 5, OP_KSQ = 6, OP_POT_RP = 7, OP_KIN2 = 8
+};
 
 template <int... Ops> struct OpL {};
 template <int... Rs> struct IL {};
@@ -252,7 +256,16 @@ struct PassArgs {
   double kscale;        // real scale folded into the kinetic factor
   double scale;         // OP_SCALE
   gb_potential pot;
-  double *partial;      // OP_KSQ: one partial sum per block
+  double *partial;      // OP_KSQ, OP_KIN2: one partial sum per block
+  // renormalisation (OP_KIN2): the last block to finish writes
+  // *sout = sqrt(ntarget / (nfactor * sum)); psi then misses that factor,
+  // which OP_POT and OP_SCALE apply when pscale points to it.  OP_KIN2 with
+  // nlast set leaves the second kinetic factor out (the last step).
+  double *sout;
+  unsigned *ndone;      // blocks finished, 0 before and after every pass
+  double ntarget, nfactor;
+  const double *pscale;
+  int nlast;
   int *errflag;         // pipelined passes: set when a bounded wait gives up
 };
 
@@ -381,7 +394,10 @@ __device__ __forceinline__ bool pot_prefetch(const PassArgs &a, unsigned o, unsi
 template <int... Ops> __host__ __device__ constexpr bool has_pot(OpL<Ops...>) {
   return ((Ops == OP_POT || Ops == OP_POT_RP) || ...);
 }
-template <int... Ops> __host__ __device__ constexpr bool has_kin(OpL<Ops...>) { return ((Ops == OP_KIN) || ...); }
+template <int... Ops> __host__ __device__ constexpr bool has_kin(OpL<Ops...>) {
+  return ((Ops == OP_KIN || Ops == OP_KIN2) || ...);
+}
+template <int... Ops> __host__ __device__ constexpr bool has_norm(OpL<Ops...>) { return ((Ops == OP_KIN2) || ...); }
 
 template <int Op, int... Rest> struct OpsHead {
   static constexpr int value = Op;
@@ -410,10 +426,10 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
     } else if constexpr (Op == OP_INV) {
       fft_line<T2, +1, N>(v, t, sm, tw);
     } else if constexpr (Op == OP_SCALE) {
-      const T s = (T) a.scale;
+      const T s = (T) (a.pscale ? a.scale * __ldg(a.pscale) : a.scale);
 #pragma unroll
       for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
-    } else if constexpr (Op == OP_KIN) {
+    } else if constexpr (Op == OP_KIN || Op == OP_KIN2) {
       // Line factor from the two other axes, times kscale; element factor
       // from the pass axis.
       int i, j, k;
@@ -425,10 +441,23 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
       const T2 f0 = ((const T2 *) a.kfac[b0])[ix0];
       const T2 f1 = ((const T2 *) a.kfac[b1])[ix1];
       T2 lf = cmul(f0, f1);
+      const T2 lf1 = lf;
       lf = cscale(lf, (T) a.kscale);
       double k2line = 0.0;
       if (a.cutoff) k2line = a.ksq[b0][ix0] + a.ksq[b1][ix1];
-      if (a.cutoff) {
+      if constexpr (Op == OP_KIN2) {
+        // the first factor carries the scale, the second does not: a forward
+        // transform would follow the inverse one and leave psi times N
+#pragma unroll
+        for (int m = 0; m < P; m++) {
+          const int p = t + TL * m;
+          const T2 fm = fa[p];
+          v[m] = cmul(v[m], cmul(lf, fm));
+          if (a.cutoff && k2line + a.ksq[ax][p] >= a.kmax2) v[m] = T2{(T) 0, (T) 0};
+          acc += (double) v[m].x * (double) v[m].x + (double) v[m].y * (double) v[m].y;
+          if (!a.nlast) v[m] = cmul(v[m], cmul(lf1, fm));
+        }
+      } else if (a.cutoff) {
 #pragma unroll
         for (int m = 0; m < P; m++) {
           const int p = t + TL * m;
@@ -447,6 +476,11 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
       unsigned vbase, vstride;
       pot_row(a, o, q, i0, j0, k0, vbase, vstride);
       const gb_potential &pt = a.pot;
+      if (a.pscale) {  // psi renormalised first
+        const T s = (T) __ldg(a.pscale);
+#pragma unroll
+        for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
+      }
       if (pot_is_simple(pt)) {
         const bool phase = (pt.c_re == 0.0);
         const double cc = phase ? pt.c_im : pt.c_re;
@@ -525,6 +559,45 @@ template <int THREADS> __device__ __forceinline__ double block_sum(double v, dou
     for (int q = 0; q < NW; q++) r += sbuf[q];
   }
   return r;
+}
+
+// Sum of the blocks' OP_KIN2 sums: every block leaves its partial, and the
+// last one to finish adds them in block order and writes the renormalisation
+// factor, so the result does not depend on which block that is and no further
+// launch is needed.  The counter wraps back to 0.
+template <int THREADS>
+__device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsigned blk, unsigned nblk) {
+  __shared__ double sbuf[THREADS % 32 ? THREADS : THREADS / 32];
+  __shared__ bool s_last;
+  // blocks of less than a warp (short lines, single columns) sum in order
+  auto sum = [&](double v) -> double {
+    if constexpr (THREADS % 32) {
+      sbuf[threadIdx.x] = v;
+      __syncthreads();
+      double t = 0.0;
+      if (threadIdx.x == 0)
+        for (int i = 0; i < THREADS; i++) t += sbuf[i];
+      return t;
+    } else {
+      return block_sum<THREADS>(v, sbuf);
+    }
+  };
+  double r = sum(acc);
+  if (threadIdx.x == 0) {
+    a.partial[blk] = r;
+    __threadfence();
+    s_last = atomicInc(a.ndone, nblk - 1) == nblk - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double s = 0.0;
+  for (unsigned i = threadIdx.x; i < nblk; i += THREADS) s += __ldcg(a.partial + i);
+  r = sum(s);
+  if (threadIdx.x == 0) {
+    const double nrm = r * a.nfactor;
+    *a.sout = nrm > 0.0 ? sqrt(a.ntarget / nrm) : 1.0;
+  }
 }
 
 // ---------------------------------------------------------------- kernels
@@ -633,6 +706,8 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, pass_min_blocks<(N / S
     T2 *d = dst + off;
 #pragma unroll
     for (int m = 0; m < P; m++) d[(unsigned) (t + TL * m) * in32] = v[m];
+    if constexpr (has_norm(OpL<Ops...>{}))
+      norm_finish<THREADS>(acc, a, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
   }
 }
 
@@ -686,6 +761,7 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, GB_PIPE_MINB)
 #pragma unroll
     for (int h = 0; h < N / ROWS; h++) tma_load_3d(land + h * ROWS * BZ, &tmap, (int) (cb * 2 * BZ), h * ROWS, (int) o, &bar);
   }
+  double acc = 0.0;
   for (unsigned it = 0; tile < ntiles; tile += gridDim.x, it++) {
     const bool ok = mbar_wait_bounded(&bar, it & 1u);
     T2 v[P];
@@ -709,12 +785,12 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, GB_PIPE_MINB)
     const unsigned o = tile / ncb;
     const unsigned q = (tile - o * ncb) * (unsigned) BZ + (unsigned) c;
     SmStrided<T2, BZ> sm{xch + c};
-    double acc = 0.0;
     Program<T, N, SmStrided<T2, BZ>, Ops...>::run(v, t, sm, a, o, q, acc);
     T2 *d = dst + (size_t) o * (size_t) N * inner + q;
 #pragma unroll
     for (int m = 0; m < P; m++) d[(unsigned) (t + TL * m) * inner] = v[m];
   }
+  if constexpr (has_norm(OpL<Ops...>{})) norm_finish<(N / Sched<N>::P) * BZ>(acc, a, blockIdx.x, gridDim.x);
 }
 
 // Launch the pipelined form when it applies (strided lines of 64..256,
@@ -768,6 +844,9 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
   constexpr size_t STAGE = has_pot(OpL<Ops...>{}) ? (size_t) Sched<N>::P * sizeof(T) : 0;
   cudaStream_t st = gb__stream();
   if (inner == 1) {
+    if constexpr (has_norm(OpL<Ops...>{})) {  // the outermost of two or more axes is never contiguous
+      return gb__set_error(1007, "fft pass: contiguous renormalising pass");
+    } else {
     using Cfg = ContigCfg<N, sizeof(T)>;
     const size_t sm = (size_t) Cfg::L * Cfg::LINE * sizeof(T2) + STAGE * Cfg::THREADS;
     auto kern = k_pass_contig<T, N, Ops...>;
@@ -779,6 +858,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
     const long nb = (outer + Cfg::L - 1) / Cfg::L;
     if (nblocks) *nblocks = nb;
     kern<<<(unsigned) nb, Cfg::THREADS, sm, st>>>((const T2 *) src, (T2 *) dst, outer, a);
+    }
   } else {
     constexpr int BZ = StridedCfg<N, sizeof(T)>::BZ;
     if (!nblocks) {

@@ -17,7 +17,7 @@ enum {
   GB_SCR_KIN2 = 6,     // kinetic factor tables of the merged K(dt) pass
   GB_SCR_CHAIN = 7,    // tile counters and ticket of the plane-chained passes
   GB_SCR_UNET = 8,     // per-chunk weight-gradient partials of the U-Net kernels
-  GB_SCR_UNETB = 9,    // packed weight operand of the U-Net tensor-core convolutions
+  GB_SCR_NORM = 9,     // renormalisation factor, counter and partial sums of the relaxation steps
   GB_SCR_COUNT = 10
 };
 
@@ -64,6 +64,9 @@ template <typename T> int gb__fft3d_t(void *data, const gb_geom *g, int sign, do
 template <typename T> int gb__split_step_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_potential *pot);
 template <typename T>
 int gb__split_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_potential *pot, int nsteps);
+template <typename T>
+int gb__relax_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const gb_potential *pot, int nsteps,
+                      double target, double step_factor);
 template <typename T> int gb__ksq_sum_t(const void *psi, void *work, const gb_geom *g, double *out);
 
 // Tensor-core U-Net convolutions (gb_unet_tc.cu): return -1 when the path is

@@ -325,7 +325,8 @@ void grid_wf_propagate_kinetic_cn(wf *gwf, REAL complex tstep) {
  * potential grid or a real external potential with g |psi|^2 may be given
  * (both NULL / g == 0 means no potential step, as grid_wf_propagate_potential
  * returns early for a NULL potential). */
-static void fused_fft_steps(wf *gwf, REAL complex time, cgrid *cpot, rgrid *vext, REAL gnl, int cutoff, int nsteps) {
+static void fused_fft_steps(wf *gwf, REAL complex time, cgrid *cpot, rgrid *vext, REAL gnl, int cutoff, int nsteps,
+                            int renormalize) {
   cgrid *grid = gwf->grid;
   const int p = psi_prec(gwf);
   gb_geom g = wf_geom(gwf);
@@ -362,11 +363,15 @@ static void fused_fft_steps(wf *gwf, REAL complex time, cgrid *cpot, rgrid *vext
     pt.g = gnl;
     has_pot = 1;
   }
-  gbh_check(gb_split_steps(gbh_dev_rw(grid->value, p), &g, &k, has_pot ? &pt : NULL, nsteps), "grid_wf_propagate");
+  if (renormalize)
+    gbh_check(gb_relax_steps(gbh_dev_rw(grid->value, p), &g, &k, &pt, nsteps, gwf->norm,
+                             gbh_step_factor(grid->nx, grid->ny, grid->nz, grid->step)),
+              "grid_wf_relax_gp_n");
+  else gbh_check(gb_split_steps(gbh_dev_rw(grid->value, p), &g, &k, has_pot ? &pt : NULL, nsteps), "grid_wf_propagate");
 }
 
 static void fused_fft_step(wf *gwf, REAL complex time, cgrid *cpot, rgrid *vext, REAL gnl, int cutoff) {
-  fused_fft_steps(gwf, time, cpot, vext, gnl, cutoff, 1);
+  fused_fft_steps(gwf, time, cpot, vext, gnl, cutoff, 1, 0);
 }
 
 /* The reference's FFT absorbing-boundary composition (src/grid_wf.c:396-422):
@@ -772,7 +777,7 @@ void grid_wf_batch_free(grid_wf_batch *bb) {
 void grid_wf_propagate_n(wf *gwf, cgrid *potential, REAL complex time, INT nsteps) {
   const int fft2 = gwf->propagator == WF_2ND_ORDER_FFT || gwf->propagator == WF_2ND_ORDER_CFFT;
   if (fft2 && !(gwf->ts_func && creal(time) != 0.0) && gwf->grid->omega == 0.0 && nsteps > 1 && nsteps < (1L << 30)) {
-    fused_fft_steps(gwf, time, potential, NULL, 0.0, gwf->propagator == WF_2ND_ORDER_CFFT, (int) nsteps);
+    fused_fft_steps(gwf, time, potential, NULL, 0.0, gwf->propagator == WF_2ND_ORDER_CFFT, (int) nsteps, 0);
     return;
   }
   for (INT s = 0; s < nsteps; s++) grid_wf_propagate(gwf, potential, time);
@@ -781,7 +786,7 @@ void grid_wf_propagate_n(wf *gwf, cgrid *potential, REAL complex time, INT nstep
 void grid_wf_propagate_gp_n(wf *gwf, rgrid *vext, REAL g, REAL complex time, INT nsteps) {
   const int fft2 = gwf->propagator == WF_2ND_ORDER_FFT || gwf->propagator == WF_2ND_ORDER_CFFT;
   if (fft2 && !(gwf->ts_func && creal(time) != 0.0) && gwf->grid->omega == 0.0 && nsteps > 1 && nsteps < (1L << 30)) {
-    fused_fft_steps(gwf, time, NULL, vext, g, gwf->propagator == WF_2ND_ORDER_CFFT, (int) nsteps);
+    fused_fft_steps(gwf, time, NULL, vext, g, gwf->propagator == WF_2ND_ORDER_CFFT, (int) nsteps, 0);
     return;
   }
   for (INT s = 0; s < nsteps; s++) grid_wf_propagate_gp(gwf, vext, g, time);
@@ -791,9 +796,19 @@ void grid_wf_propagate_gp_n(wf *gwf, rgrid *vext, REAL g, REAL complex time, INT
  * reference's callers compose grid_wf_propagate(-i dt) and grid_wf_normalize,
  * src/grid_wf.c:379-556, 681-700): nsteps of grid_wf_propagate_gp(time), each
  * followed by renormalisation to gwf->norm, with the norm reduced and applied
- * on the device, so the whole loop runs without a host synchronisation. */
+ * on the device, so the whole loop runs without a host synchronisation.  The
+ * 2nd-order FFT / CFFT propagators keep the k-space state between the steps
+ * (gb_relax_steps); a free wave function, one axis, an absorbing region in
+ * real time and Crank-Nicolson make ordinary steps. */
 void grid_wf_relax_gp_n(wf *gwf, rgrid *vext, REAL g, REAL complex time, INT nsteps) {
   cgrid *grid = gwf->grid;
+  const int fft2 = gwf->propagator == WF_2ND_ORDER_FFT || gwf->propagator == WF_2ND_ORDER_CFFT;
+  const int axes = (grid->nx > 1) + (grid->ny > 1) + (grid->nz > 1);
+  if (fft2 && (vext || g != 0.0) && axes >= 2 && !(gwf->ts_func && creal(time) != 0.0) && grid->omega == 0.0 &&
+      nsteps > 0 && nsteps < (1L << 30)) {
+    fused_fft_steps(gwf, time, NULL, vext, g, gwf->propagator == WF_2ND_ORDER_CFFT, (int) nsteps, 1);
+    return;
+  }
   for (INT s = 0; s < nsteps; s++) {
     grid_wf_propagate_gp(gwf, vext, g, time);
     const int p = psi_prec(gwf);

@@ -10,6 +10,15 @@ from libgrid_b200 import capi, workloads
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def _bind_relax(b200):
+    import ctypes as C
+
+    fn = b200.lib.grid_wf_relax_gp_n
+    fn.restype, fn.argtypes = None, [C.c_void_p, C.c_void_p, C.c_double, capi.Complex, C.c_long]
+
+
 PER, DIR = capi.WF_PERIODIC_BOUNDARY, capi.WF_DIRICHLET_BOUNDARY
 FFT2, CFFT2, CN2 = capi.WF_2ND_ORDER_FFT, capi.WF_2ND_ORDER_CFFT, capi.WF_2ND_ORDER_CN
 
@@ -105,3 +114,57 @@ def test_propagate_n_single_step_and_cn_fallback(b200):
         b200.free(w)
         b200.free(vx)
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("shape", [(32, 16, 8), (1, 64, 32), (16, 1, 128), (4, 2, 2), (128, 32, 64), (2, 256, 256),
+                                   (8, 512, 4)])
+@pytest.mark.parametrize("prec", [0, capi.GRID_PREC_FP32])
+def test_relax_matches_composition(b200, shape, prec):
+    """Relaxation steps that keep the k-space state and take the norm there
+    against propagate_gp + normalize step by step: the same to rounding (a
+    few units per transform and step: 1e-13, FP32 1e-5), for one step and
+    several, with and without an external potential."""
+    step, g, mass = 0.2, 0.01, 4.0 / workloads.GRID_AUTOAMU
+    psi0, v = workloads.gp_wells(shape, step, 0.0025, seed=31)
+    vx = b200.rgrid(*shape, step, values=50.0 * v)
+    for prop, pot, n in ((FFT2, vx, 1), (FFT2, vx, 7), (CFFT2, vx, 4), (FFT2, None, 3)):
+        outs = []
+        for merged in (True, False):
+            w = b200.wf(*shape, step, mass, PER, prop, values=psi0)
+            w.s.kmax = 9.0
+            w.s.norm = 3.0
+            if prec:
+                w.precision(prec)
+            if merged:
+                b200.lib.grid_wf_relax_gp_n(w.ptr, pot.ptr if pot else None, g, capi.Complex.of(-2j), n)
+            else:
+                for _ in range(n):
+                    w.propagate_gp(pot, g, -2j)
+                    w.normalize()
+            assert abs(w.norm() - 3.0) < (1e-12 if not prec else 1e-5)
+            outs.append(w.grid.get())
+            b200.free(w)
+        assert rel(outs[0], outs[1]) < (1e-13 if not prec else 1e-5), (prop, n)
+    b200.free(vx)
+
+
+def test_relax_other_propagators_make_ordinary_steps(b200):
+    """Crank-Nicolson and one-dimensional grids: the composition, bit for bit
+    to the norm's rounding."""
+    for shape, bc, prop in (((12, 16, 20), DIR, CN2), ((1, 1, 64), PER, FFT2)):
+        step, g, mass = 0.3, 0.001, 4.0 / workloads.GRID_AUTOAMU
+        psi0, v = workloads.cn_wells(shape, step, g)
+        outs = []
+        for merged in (True, False):
+            w = b200.wf(*shape, step, mass, bc, prop, values=psi0)
+            vx = b200.rgrid(*shape, step, values=v)
+            if merged:
+                b200.lib.grid_wf_relax_gp_n(w.ptr, vx.ptr, g, capi.Complex.of(-1j), 3)
+            else:
+                for _ in range(3):
+                    w.propagate_gp(vx, g, -1j)
+                    w.normalize()
+            outs.append(w.grid.get())
+            b200.free(w)
+            b200.free(vx)
+        assert rel(outs[0], outs[1]) < 1e-14
