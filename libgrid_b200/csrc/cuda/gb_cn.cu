@@ -9,8 +9,8 @@
 // ends; the periodic case uses the Sherman-Morrison form of
 // grid_solve_tridiagonal_system_cyclic2 (src/linalg.c:206-230).
 //
-// Fast path (no rotation, no absorbing region): every line of an axis sees
-// the same matrix, so the elimination multipliers m_i, the reciprocal pivots
+// Fast path (no absorbing region): every line of an axis sees the same matrix
+// (in a rotating frame: one matrix per perpendicular coordinate), so the elimination multipliers m_i, the reciprocal pivots
 // 1/b'_i and (periodic) the Sherman-Morrison vector z are computed once on
 // the host and each line needs only the right-hand side, one forward and one
 // backward sweep.  A CTA is one warp that owns up to 32 lines: the tile is
@@ -21,8 +21,7 @@
 // one element in shared memory so the lane-per-line accesses hit distinct
 // banks; strided (x, y) tiles hold 32 adjacent columns per row.
 //
-// General path (rotation or absorbing boundary): one thread per line with
-// per-element pivots in a global workspace laid out [i][line].
+// General path (absorbing boundary): one thread per line with per-element pivots in a global workspace laid out [i][line].
 #include <complex>
 #include <math.h>
 #include <string.h>
@@ -238,6 +237,10 @@ constexpr int kSeg = 16;
 // warp's lane-per-line accesses fall in distinct shared-memory banks.
 __host__ __device__ inline long contig_row(long n) { return (n & 1) ? n : n + 1; }
 
+// Table entries per matrix of a rotating frame's sweep: six per row, then
+// beta, 1 / gamma, 1 / den and the row's rotation coefficient.
+__host__ __device__ inline long cls_pitch(long n) { return 6 * n + 4; }
+
 // Shared-memory element (l, i) of a tile; row = padded line length
 // (contiguous) or lines per tile (strided).
 template <bool CONTIG> __device__ __forceinline__ double2 &tile_at(double2 *sm, int l, long i, long row) {
@@ -278,7 +281,11 @@ template <int SMAX, class F> __device__ __forceinline__ void seg_loop_rev(int cn
   }
 }
 
-template <bool CONTIG, int SMAX>
+// CLS: lines of different matrices (a rotating frame, whose x and y sweeps
+// carry a coefficient proportional to the perpendicular coordinate).  The
+// tables then hold one set per coordinate, a lane reads those of its line,
+// and no rows are taken from registers.
+template <bool CONTIG, int SMAX, bool CLS>
 __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ psi, CnAxis a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) uint64_t bar;
@@ -328,8 +335,22 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
     cn_tile_pot<CONTIG>(sm, (int) row, lpc, nl, line0, o, col0, a, a.pre);
   __syncthreads();
 
-  const double2 *tm = a.tab, *trb = a.tab + n, *tz = a.tab + 2 * n, *tH = a.tab + 3 * n, *tQ = a.tab + 4 * n,
-                *tG = a.tab + 5 * n;
+  const double2 *tab = a.tab;
+  double2 c3y = zero, beta = a.beta, gamma = a.gamma, den = a.den;  // gamma, den hold reciprocals
+  if constexpr (CLS) {
+    long cls = 0;
+    if (lane < nl) {
+      if (a.axis == 1) cls = CONTIG ? line0 + lane : o;
+      else if (!CONTIG) cls = (col0 + lane) / a.nz;
+    }
+    tab += cls * cls_pitch(n);
+    const double2 *sc = tab + 6 * n;
+    beta = __ldg(sc);
+    gamma = __ldg(sc + 1);
+    den = __ldg(sc + 2);
+    c3y = __ldg(sc + 3);
+  }
+  const double2 *tm = tab, *trb = tab + n, *tz = tab + 2 * n, *tH = tab + 3 * n, *tQ = tab + 4 * n, *tG = tab + 5 * n;
   const long S = (n + kSeg - 1) / kSeg;
   const long a0 = seg * S, e0 = (a0 + S < n) ? a0 + S : n;
   const int cnt = a0 < e0 ? (int) (e0 - a0) : 0;
@@ -357,8 +378,8 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
     seg_loop<SMAX>(cnt, [&](int k) {
       const long i = a0 + k;
       const double2 pp = (k + 1 < cnt) ? tile_at<CONTIG>(sm, lane, i + 1, row) : p_after;
-      const double2 b = cn_rhs(i, n, bc, a.cp, a.c2, zero, pm, p0, pp, pfirst, plast);
-      const double2 mi = (i >= klo && i <= khi) ? mc : __ldg(tm + i);
+      const double2 b = cn_rhs(i, n, bc, a.cp, a.c2, c3y, pm, p0, pp, pfirst, plast);
+      const double2 mi = (!CLS && i >= klo && i <= khi) ? mc : __ldg(tm + i);
       u = (k == 0) ? b : cs(b, cm(mi, u));
       tile_at<CONTIG>(sm, lane, i, row) = u;
       pm = p0;
@@ -386,7 +407,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
     seg_loop_rev<SMAX>(cnt, [&](int k) {
       const long i = a0 + k;
       const double2 v = ca(tile_at<CONTIG>(sm, lane, i, row), cm(__ldg(tH + i), vin));
-      const bool cst = i >= klo && i <= khi;
+      const bool cst = !CLS && i >= klo && i <= khi;
       const double2 rbi = cst ? rbc : __ldg(trb + i), qi = cst ? qc : __ldg(tQ + i);
       y = (k == cnt - 1) ? cm(rbi, v) : ca(cm(rbi, v), cm(qi, y));
       tile_at<CONTIG>(sm, lane, i, row) = y;
@@ -407,7 +428,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
       // Sherman-Morrison: fact = (x_0 + beta x_{n-1} / gamma) / den; the
       // segment holding n-1 has a zero carry-in, so x_{n-1} = y_{n-1}.
       const double2 xl = tile_at<CONTIG>(sm, lane, n - 1, row);
-      s_fact[lane] = cm(ca(xin, cm(a.beta, cm(xl, a.gamma))), a.den);  // gamma, den hold reciprocals
+      s_fact[lane] = cm(ca(xin, cm(beta, cm(xl, gamma))), den);
     }
   }
   __syncthreads();
@@ -694,7 +715,8 @@ __global__ void __launch_bounds__(kCnWarpThreads, 2) k_cn_warp(double2 *__restri
 }
 
 // General path: one thread per line, element (line, i) of a workspace array
-// at [i * nlines + line].  Handles rotation (c3) and absorbing boundaries.
+// at [i * nlines + line].  Handles absorbing boundaries, with or without
+// rotation (c3).
 __global__ void k_cn_general(double2 *__restrict__ psi, CnAxis a) {
   const long line = blockIdx.x * (long) blockDim.x + threadIdx.x;
   if (line >= a.nlines) return;
@@ -807,6 +829,58 @@ __global__ void k_cn_general(double2 *__restrict__ psi, CnAxis a) {
   } else {
     for (long i = 0; i < n; i++) psi[base + i * stride] = V[i * NL + line];
   }
+}
+
+// The tables of build_fast_tables (below) for ncls matrices, one thread each:
+// matrix k belongs to the perpendicular coordinate (k - ncls / 2) step - off
+// and has the couplings 1 -+ (c2 + c3 coordinate).
+__global__ void k_cn_class_tables(double2 *__restrict__ tab, long n, long ncls, int bc, double2 cp, double2 c2, double2 c3,
+                                  double step, double off) {
+  const long k = blockIdx.x * (long) blockDim.x + threadIdx.x;
+  if (k >= ncls) return;
+  double2 *m = tab + k * cls_pitch(n), *rb = m + n, *z = m + 2 * n, *H = m + 3 * n, *Q = m + 4 * n, *G = m + 5 * n;
+  const double2 one = make_double2(1.0, 0.0), two = make_double2(2.0, 0.0), zero = make_double2(0.0, 0.0);
+  const double2 c3y = csc(c3, (double) (k - ncls / 2) * step - off);
+  const double2 c2e = ca(c2, c3y), sup0 = ca(one, c2e), sub0 = cs(one, c2e);
+  const double2 d = cs(cp, two), gamma = make_double2(-d.x, -d.y);
+  const long S = (n + kSeg - 1) / kSeg;
+  double2 bp = bc == 3 ? cs(d, gamma) : d, h = zero, v = gamma;
+  for (long i = 0; i < n; i++) {
+    double2 mi = zero;
+    if (i > 0) {
+      const bool edge = bc != 3;
+      mi = cdiv(edge && i == n - 1 ? two : sub0, bp);
+      double2 bi = d;
+      if (bc == 3 && i == n - 1) bi = cs(d, cdiv(cm(sup0, sub0), gamma));
+      bp = cs(bi, cm(mi, edge && i == 1 ? two : sup0));
+    }
+    const double2 r = cdiv(one, bp), neg = make_double2(-mi.x, -mi.y);
+    m[i] = mi;
+    rb[i] = r;
+    const double2 q = cm(r, bc != 3 && i == 0 ? two : sup0);
+    Q[i] = make_double2(-q.x, -q.y);
+    h = i % S == 0 ? neg : cm(h, neg);
+    H[i] = h;
+    if (bc == 3) {  // right-hand side (gamma, 0, ..., 0, alpha), eliminated
+      if (i > 0) v = cs(i == n - 1 ? sup0 : zero, cm(mi, v));
+      z[i] = v;
+    }
+  }
+  double2 g = zero, x = zero;
+  for (long i = n - 1; i >= 0; i--) {
+    g = (i == n - 1 || i % S == S - 1) ? Q[i] : cm(Q[i], g);
+    G[i] = g;
+    if (bc == 3) {
+      x = i == n - 1 ? cm(z[i], rb[i]) : cm(cs(z[i], cm(sup0, x)), rb[i]);
+      z[i] = x;
+    }
+  }
+  double2 *sc = m + 6 * n;
+  const double2 ig = cdiv(one, gamma);
+  sc[0] = sub0;
+  sc[1] = ig;
+  sc[2] = bc == 3 ? cdiv(one, ca(ca(one, z[0]), cm(cm(sub0, z[n - 1]), ig))) : one;
+  sc[3] = c3y;
 }
 
 // Host-side uniform tables for one axis: m, 1/b', z (periodic), and the
@@ -950,8 +1024,10 @@ struct CnCacheEntry {
 static CnCacheEntry g_cn_cache[3];
 static void *g_cn_tab_base = nullptr;
 
+constexpr long kFastMaxN = 4096;  // longest line of the fast path
+
 static double2 *fast_tables(int slot, long n, int bc, cd cp, cd c2, int nseg, cudaStream_t st, CnAxis *a) {
-  const long nmax = 4096;
+  const long nmax = kFastMaxN;
   if (n > nmax) {
     gb__set_error(1013, "cn: line length above 4096");
     return nullptr;
@@ -988,6 +1064,39 @@ static double2 *fast_tables(int slot, long n, int bc, cd cp, cd c2, int nseg, cu
   a->mc = e.ft.mc;
   a->rbc = e.ft.rbc;
   a->qc = e.ft.qc;
+  return tab;
+}
+
+// Tables of a rotating frame's sweep, built on the device when the parameters
+// change (one kernel of a thread per matrix).
+struct CnClassKey {
+  double2 *base;
+  long n, ncls;
+  int bc;
+  cd cp, c2, c3;
+  double step, off;
+};
+static CnClassKey g_cls_key[2];
+
+static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off,
+                             cudaStream_t st) {
+  double2 *tab = (double2 *) gb__scratch(axis == 0 ? GB_SCR_CNROT0 : GB_SCR_CNROT1,
+                                         sizeof(double2) * (size_t) (cls_pitch(n) * ncls));
+  if (!tab) return nullptr;
+  CnClassKey &k = g_cls_key[axis];
+  if (k.base == tab && k.n == n && k.ncls == ncls && k.bc == bc && k.cp == cp && k.c2 == c2 && k.c3 == c3 &&
+      k.step == step && k.off == off)
+    return tab;
+  auto v2 = [](cd z) { return make_double2(z.real(), z.imag()); };
+  k_cn_class_tables<<<(unsigned) ((ncls + 31) / 32), 32, 0, st>>>(tab, n, ncls, bc, v2(cp), v2(c2), v2(c3), step, off);
+  gb__count_launch();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaGetLastError() != cudaSuccess || cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    gb__set_error(3, "cn class tables");
+    return nullptr;
+  }
+  // a captured kernel has not run: the tables count as built only by one that has
+  k = cap == cudaStreamCaptureStatusNone ? CnClassKey{tab, n, ncls, bc, cp, c2, c3, step, off} : CnClassKey{};
   return tab;
 }
 
@@ -1066,13 +1175,13 @@ static int launch_cn_warp(void *psi, CnAxis &a, bool contig, int axis, cudaStrea
 // 0.487 ms per step); -1 only queries.
 // The fast kernel unrolled for the segment length of lines of n points.
 using FastKernel = void (*)(double2 *, CnAxis);
-template <bool CONTIG> static FastKernel fast_kernel(long n) {
+template <bool CONTIG, bool CLS> static FastKernel fast_kernel(long n) {
   const long S = (n + kSeg - 1) / kSeg;
-  if (S <= 4) return k_cn_fast<CONTIG, 4>;
-  if (S <= 8) return k_cn_fast<CONTIG, 8>;
-  if (S <= 12) return k_cn_fast<CONTIG, 12>;
-  if (S <= 16) return k_cn_fast<CONTIG, 16>;
-  return k_cn_fast<CONTIG, 0>;
+  if (S <= 4) return k_cn_fast<CONTIG, 4, CLS>;
+  if (S <= 8) return k_cn_fast<CONTIG, 8, CLS>;
+  if (S <= 12) return k_cn_fast<CONTIG, 12, CLS>;
+  if (S <= 16) return k_cn_fast<CONTIG, 16, CLS>;
+  return k_cn_fast<CONTIG, 0, CLS>;
 }
 
 static int g_cn_warp_on = 0;
@@ -1090,7 +1199,6 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
   cudaStream_t st = gb__stream();
   const cd c = cd(0.0, 4.0) * p->mass * g->step * g->step / 1.0;  // 4 i m h^2 / hbar (hbar = 1)
   const cd tstep(p->tstep_re, p->tstep_im);
-  const bool fast = (p->omega == 0.0) && !p->absorb;
   const long nxyz = g->nx * g->ny * g->nz;
   gb_potential none;
   memset(&none, 0, sizeof(none));
@@ -1157,7 +1265,14 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
     a.pre = (s == 0) ? *prep : none_pot;
     a.post = (s == na - 1) ? *postp : none_pot;
 
-    if (fast && a.n <= 32 * kLaneSegMax && g_cn_warp_on) {
+    // in a rotating frame the matrix of an x (y) line depends on its y (x)
+    const bool cls = c3 != cd(0.0);
+    // a rotating frame goes on to the general path where the tiles or the
+    // tables (up to 1 GB) of the fast one end; without rotation those are errors
+    const long ncls = axis == 0 ? g->ny : g->nx;
+    const bool fast = !p->absorb && (p->omega == 0.0 || (a.n <= kFastMaxN && (contig || a.outer <= 65535) &&
+                                                         (!cls || cls_pitch(a.n) * ncls <= (1L << 26))));
+    if (fast && !cls && a.n <= 32 * kLaneSegMax && g_cn_warp_on) {
       const cd cp = c / tstep;
       double2 *tab = fast_tables(s, a.n, p->boundary, cp, c2, 32, st, &a);
       if (!tab) return gb_last_error();
@@ -1166,7 +1281,9 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
       GB_TRYC(launch_cn_warp(psi, a, contig, axis, st));
     } else if (fast) {
       const cd cp = c / tstep;
-      double2 *tab = fast_tables(s, a.n, p->boundary, cp, c2, kSeg, st, &a);
+      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step,
+                                        a.coord_off, st)
+                         : fast_tables(s, a.n, p->boundary, cp, c2, kSeg, st, &a);
       if (!tab) return gb_last_error();
       a.tab = tab;
       a.cp = make_double2(cp.real(), cp.imag());
@@ -1178,8 +1295,8 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&smpm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         cudaFuncAttributes fa0, fa1;
-        cudaFuncGetAttributes(&fa0, k_cn_fast<true, 0>);
-        cudaFuncGetAttributes(&fa1, k_cn_fast<false, 0>);
+        cudaFuncGetAttributes(&fa0, k_cn_fast<true, 0, false>);
+        cudaFuncGetAttributes(&fa1, k_cn_fast<false, 0, false>);
         const size_t st_max = fa0.sharedSizeBytes > fa1.sharedSizeBytes ? fa0.sharedSizeBytes : fa1.sharedSizeBytes;
         const long b = (long) smpm / 2 - 1024 - (long) st_max;
         budget = b > 16 * 1024 ? (size_t) b : 16 * 1024;
@@ -1191,7 +1308,7 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         if (lpc < 1) return gb__set_error(1011, "cn: line too long for a shared-memory tile");
         a.lpc = (int) lpc;
         const size_t sm = (size_t) lpc * row * 16;
-        const FastKernel kern = fast_kernel<true>(a.n);
+        const FastKernel kern = cls ? fast_kernel<true, true>(a.n) : fast_kernel<true, false>(a.n);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         const long nb = (a.outer + lpc - 1) / lpc;
         {
@@ -1209,7 +1326,7 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         const long lpc = pow2_at_most(cap);
         a.lpc = (int) lpc;
         const size_t sm = (size_t) lpc * a.n * 16;
-        const FastKernel kern = fast_kernel<false>(a.n);
+        const FastKernel kern = cls ? fast_kernel<false, true>(a.n) : fast_kernel<false, false>(a.n);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         if (a.outer > 65535) return gb__set_error(1012, "cn: outer extent above 65535");
         dim3 grid((unsigned) ((a.inner + lpc - 1) / lpc), (unsigned) a.outer);

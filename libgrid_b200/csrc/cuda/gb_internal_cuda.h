@@ -18,7 +18,9 @@ enum {
   GB_SCR_CHAIN = 7,    // tile counters and ticket of the plane-chained passes
   GB_SCR_UNET = 8,     // per-chunk weight-gradient partials of the U-Net kernels
   GB_SCR_NORM = 9,     // renormalisation factor, counter and partial sums of the relaxation steps
-  GB_SCR_COUNT = 10
+  GB_SCR_CNROT0 = 10,  // line-solver tables of a rotating frame's x sweep
+  GB_SCR_CNROT1 = 11,  // and of its y sweep
+  GB_SCR_COUNT = 12
 };
 
 void *gb__scratch(int slot, size_t bytes);

@@ -269,6 +269,24 @@ def test_cn_rotation_and_absorber(b200, restate, bc):
 
 
 @pytest.mark.parametrize("bc", [DIR, NEU, PER])
+@pytest.mark.parametrize("shape", [(16, 12, 10), (33, 70, 7), (20, 41, 1), (40, 2, 65), (2, 100, 3), (1, 24, 9)])
+def test_cn_rotation(b200, restate, bc, shape):
+    """Rotating frame without an absorber: one matrix per perpendicular
+    coordinate (tiles that span several of them, partial tiles, contiguous
+    lines in two dimensions), with a moving frame on top."""
+    step, mass, k0 = 0.3, 1.0, (0.1, -0.2, 0.05)
+    rng = np.random.default_rng(29)
+    psi0 = smooth_state(shape, step) + 0.01 * rand_c(rng, shape)
+    v = 0.02 * rng.standard_normal(shape).astype(complex)
+    for time in (0.05, -0.1j):
+        got = b200_cn_run(b200, psi0, v, step, mass, time, bc, 3, k0, omega=0.3)
+        want = psi0.copy()
+        for _ in range(3):
+            want = restate.cn_step(want, step, mass, time, bc, k0=k0, omega=0.3, vc=v)
+        assert rel(got, want) < TOL_PSI
+
+
+@pytest.mark.parametrize("bc", [DIR, NEU, PER])
 @pytest.mark.parametrize("shape", [(16, 192, 200), (256, 4, 33)])
 def test_cn_line_solvers_agree(b200, bc, shape):
     """The warp-cooperative line solver (lines up to 256 points, segment
