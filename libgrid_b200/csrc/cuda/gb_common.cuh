@@ -176,6 +176,38 @@ extern "C" cudaStream_t gb__stream(void);
   } while (0)
 
 // ------------------------------------------------------------------------
+// Launches whose start overlaps the end of the kernel before them on the
+// stream (programmatic dependent launch).  Every CTA of such a kernel calls
+// grid_wait on each pointer it reads before it touches global memory: it
+// returns when the kernels before have finished and their writes are visible.
+// The pointer passes through the statement, so that no load of it, a read-only
+// one of a restrict pointer included, can be moved above.  The next launch is
+// let go right after, when all CTAs of this one have started.  For the line
+// passes, launch by launch / overlapped: a 32^3 step (nine passes) 38.9 / 23.2
+// us, a 128^3 convolution 135 / 117 us, ten relaxation steps at 128^3 909 / 822
+// us, a 256^3 step 888 / 889 us (FP64).
+template <typename P> __device__ __forceinline__ void grid_wait(P &p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+inline void launch_overlapped(void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                              Args... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, Params(args)...);  // the caller checks the launch
+}
+
+// ------------------------------------------------------------------------
 // Bulk asynchronous copies (TMA, non-tensor form) and mbarriers.
 // All waits are bounded: after GB_WAIT_LIMIT polls the caller gets `false`
 // and must record an error and leave without touching the data.

@@ -472,7 +472,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
     } else if constexpr (Op == OP_INV) {
       fft_line<T2, +1, N>(v, t, sm, tw);
     } else if constexpr (Op == OP_SCALE) {
-      const T s = (T) (a.pscale ? a.scale * __ldg(a.pscale) : a.scale);
+      const T s = (T) (a.pscale ? a.scale * __ldcg(a.pscale) : a.scale);
 #pragma unroll
       for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
     } else if constexpr (Op == OP_KIN || Op == OP_KIN2) {
@@ -523,7 +523,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
       pot_row(a, o, q, i0, j0, k0, vbase, vstride);
       const gb_potential &pt = a.pot;
       if (a.pscale) {  // psi renormalised first
-        const T s = (T) __ldg(a.pscale);
+        const T s = (T) __ldcg(a.pscale);
 #pragma unroll
         for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
       }
@@ -683,6 +683,7 @@ __global__ void __launch_bounds__(ContigCfg<N, sizeof(T)>::THREADS, ContigCfg<N,
   const int l = threadIdx.x / TL;
   const unsigned line = blockIdx.x * (unsigned) Cfg::L + (unsigned) l;
   const bool ok = line < (unsigned long) nlines;
+  grid_wait(src);
   const T2 *s = src + (size_t) line * N;
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, pass_min_blocks<(N / S
   // element (line, t + TL m) sits at base + (t + TL m) * inner; the whole
   // grid has fewer than 2^31 points, so the in-tile offsets fit 32 bits
   const size_t off = (size_t) o * (size_t) N * (size_t) inner + q;
+  grid_wait(src);
   const T2 *s = src + off;
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
@@ -791,6 +793,7 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, GB_PIPE_MINB)
   T2 *xch = (T2 *) (base + TILE_BYTES);
   const int tid = threadIdx.x;
   const int c = tid % BZ, t = tid / BZ;
+  grid_wait(dst);
   // a descriptor that is not 64-byte aligned is recorded (code 3) and the
   // pass skipped
   if (((size_t) &tmap & 63u) != 0) {
@@ -876,8 +879,8 @@ int launch_strided_pipe(const void *src, void *dst, const PassArgs &a, long oute
     CUtensorMap tm;
     if (gb__tmap_lines(&tm, src, outer, N, inner, sizeof(T) == 4, BZ, pipe_rows<N>())) return gb_last_error();
     const long g = ntiles < rgrid ? ntiles : rgrid;
-    kern<<<(unsigned) g, THREADS, SM, gb__stream()>>>((T2 *) dst, (unsigned) inner, (unsigned) ncb,
-                                                       (unsigned) ntiles, a, tm);
+    launch_overlapped(kern, dim3((unsigned) g), THREADS, SM, gb__stream(), (T2 *) dst, (unsigned) inner, (unsigned) ncb,
+                      (unsigned) ntiles, a, tm);
     *launched = 1;
     GB_CHECK_LAUNCH("pipelined fft pass");
     return 0;
@@ -905,7 +908,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
     }
     const long nb = (outer + Cfg::L - 1) / Cfg::L;
     if (nblocks) *nblocks = nb;
-    kern<<<(unsigned) nb, Cfg::THREADS, sm, st>>>((const T2 *) src, (T2 *) dst, outer, a);
+    launch_overlapped(kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst, outer, a);
     }
   } else {
     constexpr int BZ = StridedCfg<N, sizeof(T)>::BZ;
@@ -924,7 +927,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) (inner / BZ), (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      kern<<<grid, (N / Sched<N>::P) * BZ, sm, st>>>((const T2 *) src, (T2 *) dst, inner, a);
+      launch_overlapped(kern, grid, (N / Sched<N>::P) * BZ, sm, st, (const T2 *) src, (T2 *) dst, inner, a);
     } else if (outer <= 65535) {
       const size_t sm = (size_t) N * sizeof(T2) + STAGE * (N / Sched<N>::P);
       auto kern = k_pass_strided<T, N, 1, Ops...>;
@@ -935,7 +938,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) inner, (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      kern<<<grid, N / Sched<N>::P, sm, st>>>((const T2 *) src, (T2 *) dst, inner, a);
+      launch_overlapped(kern, grid, N / Sched<N>::P, sm, st, (const T2 *) src, (T2 *) dst, inner, a);
     } else {
       return gb__set_error(1001, "fft pass: outer extent above 65535");
     }
