@@ -7,11 +7,9 @@
 // lands outside the grid again (the reference recurses without end there);
 // this implementation uses the single plane instead.
 //
-// Each output column (j, k) is one thread of a CTA whose 8 x 32 (y, z) tile
-// marches along a chunk of x planes (k_fd below): x neighbours in registers,
-// y/z neighbours from a shared-memory plane with a one-point halo, so every
-// input element is read from HBM about once.  Laplacian sums keep the
-// reference's left-to-right order
+// Stencils read their neighbours directly, one output element per thread and
+// load batch (k_fd below).  Laplacian sums keep the reference's left-to-right
+// order
 //   (-6 c + z+ + z- + y+ + y- + x+ + x-) / h^2     (src/cgrid_diff.c:330-335).
 #include <string.h>
 
@@ -75,6 +73,97 @@ __device__ __forceinline__ typename Elem<T, REAL>::V fetch(const typename Elem<T
   return src[(i * a.ny + j) * a.row + k];
 }
 
+// Direct stencils.  Bound by memory: a CTA takes kFdThreads * U consecutive
+// elements, a thread U of them kFdThreads apart with their loads issued
+// together.  A chunk's row and plane neighbours are the chunk itself, its edge
+// rows and two planes nearby, so DRAM sees each element about once.  Halo tiles
+// marched along x (k_fd_kinetic below keeps them) hold two planes of a column
+// in flight and meet at a CTA barrier once per plane.  Tiles / direct, FP64, in
+// microseconds: complex gradients 150 / 81 at 256^3, 46 / 17 at 200 x 150 x
+// 101, 16.7 / 5.4 at 64^3; complex Laplacian 152 / 135, 48.7 / 28.3, 17.5 /
+// 5.5; real Laplacian 118 / 83, 37 / 19, 14.6 / 5.1.  Not kept: the boundary as
+// an index select instead of a branch (complex Laplacian at 256^3 167), chunks
+// of two planes (138, real 117).
+constexpr int kFdThreads = 256;
+
+// The axis neighbour of element idx at coordinate c of an axis of n points
+// with element stride s: in range at once, else by the boundary rule
+// (src/cgrid_bc.c:21-86).  A Neumann axis of length 1 uses its single plane.
+template <int DIR, typename T, bool REAL, typename I>
+__device__ __forceinline__ typename Elem<T, REAL>::V neighbour(const typename Elem<T, REAL>::V *__restrict__ src, I idx,
+                                                               I c, I n, I s, const FdArgs &a) {
+  const bool in = DIR > 0 ? c + 1 < n : c > 0;
+  if (in) return src[DIR > 0 ? idx + s : idx - s];
+  if (a.bc == GB_BC_DIRICHLET) return Elem<T, REAL>::outside(a.out_re, a.out_im);
+  I m;  // the coordinate that stands for the outside one
+  if (a.bc == GB_BC_PERIODIC) m = DIR > 0 ? 0 : n - 1;
+  else m = n == 1 ? 0 : DIR > 0 ? n - 2 : 1;
+  return src[idx - c * s + m * s];
+}
+
+// Element e of the grid's nx * ny * nz points: its storage index and its
+// neighbours along the axes that MODE takes (0, 1, 2: x, y, z; 3: all, in the
+// order z+, z-, y+, y-, x+, x-).
+template <typename T, bool REAL, int MODE, typename I>
+__device__ __forceinline__ I fd_load(typename Elem<T, REAL>::V (&nb)[MODE == 3 ? 6 : 2],
+                                     const typename Elem<T, REAL>::V *__restrict__ src, I e, const FdArgs &a) {
+  constexpr int Y = MODE == 3 ? 2 : 0, X = MODE == 3 ? 4 : 0;
+  const I nz = (I) a.nz, ny = (I) a.ny, r = e / nz, k = e - r * nz, i = r / ny, j = r - i * ny;
+  const I sy = (I) a.row, sx = (I) a.ny * (I) a.row, idx = r * sy + k;
+  if constexpr (MODE >= 2) {
+    nb[0] = neighbour<1, T, REAL, I>(src, idx, k, nz, (I) 1, a);
+    nb[1] = neighbour<-1, T, REAL, I>(src, idx, k, nz, (I) 1, a);
+  }
+  if constexpr (MODE == 1 || MODE == 3) {
+    nb[Y] = neighbour<1, T, REAL, I>(src, idx, j, ny, sy, a);
+    nb[Y + 1] = neighbour<-1, T, REAL, I>(src, idx, j, ny, sy, a);
+  }
+  if constexpr (MODE == 0 || MODE == 3) {
+    nb[X] = neighbour<1, T, REAL, I>(src, idx, i, (I) a.nx, sx, a);
+    nb[X + 1] = neighbour<-1, T, REAL, I>(src, idx, i, (I) a.nx, sx, a);
+  }
+  return idx;
+}
+
+__host__ __device__ constexpr int fd_unroll(int mode) { return mode == 3 ? 2 : 4; }
+
+// MODE 0, 1, 2: second difference (lap) or central difference along x, y, z;
+// MODE 3: the seven-point Laplacian.
+template <typename T, bool REAL, int MODE, typename I>
+__global__ void __launch_bounds__(kFdThreads) k_fd(bool lap, typename Elem<T, REAL>::V *__restrict__ dst,
+                                                   const typename Elem<T, REAL>::V *__restrict__ src, FdArgs a) {
+  using E = Elem<T, REAL>;
+  using V = typename E::V;
+  constexpr int U = fd_unroll(MODE), NB = MODE == 3 ? 6 : 2;
+  const I total = (I) a.nx * (I) a.ny * (I) a.nz;
+  const I e0 = (I) blockIdx.x * (I) (kFdThreads * U) + (I) threadIdx.x;
+  const bool centre = MODE == 3 || lap;
+  V c[U], nb[U][NB];
+  I idx[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const I e = e0 + (I) (u * kFdThreads);
+    if (e < total) {
+      idx[u] = fd_load<T, REAL, MODE, I>(nb[u], src, e, a);
+      if (centre) c[u] = src[idx[u]];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    if (e0 + (I) (u * kFdThreads) < total) {
+      V r;
+      if (centre) {
+        r = E::scale(c[u], (T) (MODE == 3 ? -6.0 : -2.0));
+#pragma unroll
+        for (int q = 0; q < NB; q++) r = E::add(r, nb[u][q]);
+      } else {
+        r = E::sub(nb[u][0], nb[u][1]);
+      }
+      dst[idx[u]] = E::scale(r, (T) a.coef);
+    }
+  }
+}
+
 // Tiles: a CTA of 256 threads owns a (kFdTY x kFdTZ) = (8 x 32) tile of
 // (y, z) over kFdXC consecutive x planes and marches along x.  Each thread
 // keeps its own column's x-1, x and x+1 values in registers and loads the
@@ -86,7 +175,8 @@ __device__ __forceinline__ typename Elem<T, REAL>::V fetch(const typename Elem<T
 // warp 1 the row y+8, warp 2 the columns z-1 (lanes 0-7) and z+32 (lanes
 // 8-15).  Measured at 256^3: two planes ahead at four CTAs per SM beat four
 // planes ahead at three.
-constexpr int kFdTY = 8, kFdTZ = 32, kFdXC = 16, kFdThreads = kFdTY * kFdTZ;
+constexpr int kFdTY = 8, kFdTZ = 32, kFdXC = 16;
+static_assert(kFdTY * kFdTZ == kFdThreads, "one thread per tile column");
 
 template <typename T, bool REAL> struct FdTile {
   using E = Elem<T, REAL>;
@@ -137,58 +227,33 @@ template <typename T, bool REAL> struct FdTile {
   }
 };
 
-template <typename T, bool REAL>
-__global__ void __launch_bounds__(kFdThreads, 4) k_fd(int op, typename Elem<T, REAL>::V *__restrict__ dst,
-                                                   const typename Elem<T, REAL>::V *__restrict__ src, FdArgs a) {
-  using E = Elem<T, REAL>;
-  using V = typename E::V;
-  __shared__ V sm[2][kFdTY + 2][kFdTZ + 2];
-  const int tz = threadIdx.x % kFdTZ, ty = threadIdx.x / kFdTZ;
-  const long k = blockIdx.x * (long) kFdTZ + tz, j = blockIdx.y * (long) kFdTY + ty;
-  const long i0 = blockIdx.z * (long) kFdXC;
-  const long i1 = i0 + kFdXC < a.nx ? i0 + kFdXC : a.nx;
-  const bool in = k < a.nz && j < a.ny;
-  const T coef = (T) a.coef;
-  FdTile<T, REAL> t;
-  t.init(src, a, i0, j, k, ty, tz);
-  V *out = dst + (i0 * a.ny + j) * a.row + k;
-  const long pstride = a.ny * a.row;
-  for (long i = i0; i < i1; i++) {
-    const V hq = t.prefetch(src, a, i, i1, j, k);
-    const int b = (int) ((i - i0) & 1);
-    const V c = t.c, xm = t.xm, xp = t.xp;
-    sm[b][ty + 1][tz + 1] = c;
-    if (t.has_h) sm[b][t.hy][t.hz] = t.h;
-    __syncthreads();
-    const V zp = sm[b][ty + 1][tz + 2], zm = sm[b][ty + 1][tz];
-    const V yp = sm[b][ty + 2][tz + 1], ym = sm[b][ty][tz + 1];
-    V r;
-    switch (op) {
-      case GB_FD_LAPLACE: {
-        V s = E::scale(c, (T) -6.0);
-        s = E::add(s, zp);
-        s = E::add(s, zm);
-        s = E::add(s, yp);
-        s = E::add(s, ym);
-        s = E::add(s, xp);
-        s = E::add(s, xm);
-        r = E::scale(s, coef);
-      } break;
-      case GB_FD_LAPLACE_X: r = E::scale(E::add(E::add(E::scale(c, (T) -2.0), xp), xm), coef); break;
-      case GB_FD_LAPLACE_Y: r = E::scale(E::add(E::add(E::scale(c, (T) -2.0), yp), ym), coef); break;
-      case GB_FD_LAPLACE_Z: r = E::scale(E::add(E::add(E::scale(c, (T) -2.0), zp), zm), coef); break;
-      case GB_FD_GRADIENT_X: r = E::scale(E::sub(xp, xm), coef); break;
-      case GB_FD_GRADIENT_Y: r = E::scale(E::sub(yp, ym), coef); break;
-      default: r = E::scale(E::sub(zp, zm), coef); break;
+// sum of a CTA's (sx, sy) by a fixed shuffle tree and warp order
+__device__ __forceinline__ void fd_block_sum(double sx, double sy, double2 *out) {
+  __shared__ double sb[2 * kFdThreads / 32];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    sx += __shfl_down_sync(0xffffffffu, sx, off);
+    sy += __shfl_down_sync(0xffffffffu, sy, off);
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) {
+    sb[2 * w] = sx;
+    sb[2 * w + 1] = sy;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double tx = 0.0, tyy = 0.0;
+    for (int q = 0; q < kFdThreads / 32; q++) {
+      tx += sb[2 * q];
+      tyy += sb[2 * q + 1];
     }
-    if (in) out[(i - i0) * pstride] = r;
-    t.shift(hq);
+    *out = make_double2(tx, tyy);
   }
 }
 
 // sum conj(psi) * Laplacian(psi) over the grid, the Laplacian summed in the
 // stencil kernel's order and scaled by 1/h^2 (a.coef) before the product.
-// Same tiles and march as k_fd; each CTA writes one partial (x, y) sum,
+// Each CTA writes one partial (x, y) sum,
 // reduced in a fixed order, so the result is the same from run to run.
 template <typename T>
 __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic(const C2<T> *__restrict__ src, FdArgs a,
@@ -196,7 +261,6 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic(const C2<T> *__restri
   using E = Elem<T, false>;
   using V = C2<T>;
   __shared__ V sm[2][kFdTY + 2][kFdTZ + 2];
-  __shared__ double sb[2 * kFdThreads / 32];
   const int tz = threadIdx.x % kFdTZ, ty = threadIdx.x / kFdTZ;
   const long k = blockIdx.x * (long) kFdTZ + tz, j = blockIdx.y * (long) kFdTY + ty;
   const long i0 = blockIdx.z * (long) kFdXC;
@@ -228,25 +292,47 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic(const C2<T> *__restri
     }
     t.shift(hq);
   }
+  fd_block_sum(sx, sy, partial + ((long) blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+}
+
+// The same sum with direct neighbour reads, for grids that L2 holds: CTAs walk
+// the chunks with a stride of the launch.  Energy call, tiles / direct: 100 / 78
+// us at 200 x 150 x 101 (48 MB of psi); 259 / 271 us at 256^3 (268 MB), where
+// L2 no longer holds what is read again.
+constexpr int kFdKinBlocks = 148 * 6;
+constexpr long kFdKinDirectBytes = 64L << 20;
+
+template <typename T>
+__global__ void __launch_bounds__(kFdThreads) k_fd_kinetic_direct(const C2<T> *__restrict__ src, FdArgs a,
+                                                                  double2 *__restrict__ partial) {
+  constexpr unsigned U = 2;
+  const unsigned total = (unsigned) (a.nx * a.ny * a.nz);
+  double sx = 0.0, sy = 0.0;
+  for (unsigned e0 = blockIdx.x * (kFdThreads * U) + threadIdx.x; e0 < total; e0 += gridDim.x * (kFdThreads * U)) {
+    C2<T> c[U], nb[U][6];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    sx += __shfl_down_sync(0xffffffffu, sx, off);
-    sy += __shfl_down_sync(0xffffffffu, sy, off);
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) {
-    sb[2 * w] = sx;
-    sb[2 * w + 1] = sy;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tx = 0.0, tyy = 0.0;
-    for (int q = 0; q < kFdThreads / 32; q++) {
-      tx += sb[2 * q];
-      tyy += sb[2 * q + 1];
+    for (unsigned u = 0; u < U; u++) {
+      const unsigned e = e0 + u * kFdThreads;
+      if (e < total) c[u] = src[fd_load<T, false, 3, unsigned>(nb[u], src, e, a)];
     }
-    partial[((long) blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = make_double2(tx, tyy);
+#pragma unroll
+    for (unsigned u = 0; u < U; u++) {
+      if (e0 + u * kFdThreads < total) {
+        double sr = -6.0 * (double) c[u].x, si = -6.0 * (double) c[u].y;
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+          sr += (double) nb[u][q].x;
+          si += (double) nb[u][q].y;
+        }
+        sr *= a.coef;
+        si *= a.coef;
+        // conj(c) * (sr + i si)
+        sx += (double) c[u].x * sr + (double) c[u].y * si;
+        sy += (double) c[u].x * si - (double) c[u].y * sr;
+      }
+    }
   }
+  fd_block_sum(sx, sy, partial + blockIdx.x);
 }
 
 // Sum of n partials by one CTA of 256 threads: strided per-thread sums,
@@ -287,6 +373,31 @@ int fd_grid(const gb_geom *g, dim3 *grid) {
   return 0;
 }
 
+// 32-bit indices up to 2^31 stored elements less the overhang of a launch: the
+// two divisions of a point cost several times as much in 64 bits.
+template <typename T, bool REAL, int MODE>
+int fd_launch(bool lap, void *dst, const void *src, const FdArgs &a) {
+  using V = typename Elem<T, REAL>::V;
+  const long per = (long) kFdThreads * fd_unroll(MODE), nb = (a.nx * a.ny * a.nz + per - 1) / per;
+  const bool w32 = a.nx * a.ny * a.row < (1L << 31) - (1L << 20);
+  auto kern = w32 ? k_fd<T, REAL, MODE, unsigned> : k_fd<T, REAL, MODE, unsigned long>;
+  kern<<<(unsigned) nb, kFdThreads, 0, gb__stream()>>>(lap, (V *) dst, (const V *) src, a);
+  GB_CHECK_LAUNCH("fd stencil");
+  return 0;
+}
+
+template <typename T, bool REAL> int fd_op(int op, void *dst, const void *src, const FdArgs &a) {
+  switch (op) {
+    case GB_FD_LAPLACE: return fd_launch<T, REAL, 3>(true, dst, src, a);
+    case GB_FD_LAPLACE_X: return fd_launch<T, REAL, 0>(true, dst, src, a);
+    case GB_FD_LAPLACE_Y: return fd_launch<T, REAL, 1>(true, dst, src, a);
+    case GB_FD_LAPLACE_Z: return fd_launch<T, REAL, 2>(true, dst, src, a);
+    case GB_FD_GRADIENT_X: return fd_launch<T, REAL, 0>(false, dst, src, a);
+    case GB_FD_GRADIENT_Y: return fd_launch<T, REAL, 1>(false, dst, src, a);
+    default: return fd_launch<T, REAL, 2>(false, dst, src, a);
+  }
+}
+
 }  // namespace
 
 extern "C" int gb_fd(int op, void *dst, const void *src, const gb_geom *g, int bc, double out_re, double out_im, double coef,
@@ -302,16 +413,8 @@ extern "C" int gb_fd(int op, void *dst, const void *src, const gb_geom *g, int b
   a.coef = coef;
   dim3 grid;
   if (fd_grid(g, &grid)) return gb_last_error();
-  cudaStream_t st = gb__stream();
-  if (is_real) {
-    if (g->prec == GB_FP32) k_fd<float, true><<<grid, kFdThreads, 0, st>>>(op, (float *) dst, (const float *) src, a);
-    else k_fd<double, true><<<grid, kFdThreads, 0, st>>>(op, (double *) dst, (const double *) src, a);
-  } else {
-    if (g->prec == GB_FP32) k_fd<float, false><<<grid, kFdThreads, 0, st>>>(op, (float2 *) dst, (const float2 *) src, a);
-    else k_fd<double, false><<<grid, kFdThreads, 0, st>>>(op, (double2 *) dst, (const double2 *) src, a);
-  }
-  GB_CHECK_LAUNCH("fd stencil");
-  return 0;
+  if (is_real) return g->prec == GB_FP32 ? fd_op<float, true>(op, dst, src, a) : fd_op<double, true>(op, dst, src, a);
+  return g->prec == GB_FP32 ? fd_op<float, false>(op, dst, src, a) : fd_op<double, false>(op, dst, src, a);
 }
 
 extern "C" int gb_fd_kinetic_sum(const void *psi, const gb_geom *g, int bc, double out_re, double out_im, double inv_h2,
@@ -327,12 +430,17 @@ extern "C" int gb_fd_kinetic_sum(const void *psi, const gb_geom *g, int bc, doub
   a.coef = inv_h2;
   dim3 grid;
   if (fd_grid(g, &grid)) return gb_last_error();
-  const long nb = (long) grid.x * grid.y * grid.z;
+  const long n = g->nx * g->ny * g->nz, chunks = (n + 2 * kFdThreads - 1) / (2 * kFdThreads);
+  const bool direct = n * (g->prec == GB_FP32 ? 8 : 16) <= kFdKinDirectBytes;
+  const long nb = !direct ? (long) grid.x * grid.y * grid.z : chunks < kFdKinBlocks ? chunks : kFdKinBlocks;
   double2 *partial = (double2 *) gb__scratch(GB_SCR_PARTIAL, sizeof(double2) * (size_t) nb);
   double2 *res = (double2 *) gb__result_slot();
   if (!partial || !res) return gb_last_error();
   cudaStream_t st = gb__stream();
-  if (g->prec == GB_FP32) k_fd_kinetic<float><<<grid, kFdThreads, 0, st>>>((const float2 *) psi, a, partial);
+  if (direct) {
+    if (g->prec == GB_FP32) k_fd_kinetic_direct<float><<<(unsigned) nb, kFdThreads, 0, st>>>((const float2 *) psi, a, partial);
+    else k_fd_kinetic_direct<double><<<(unsigned) nb, kFdThreads, 0, st>>>((const double2 *) psi, a, partial);
+  } else if (g->prec == GB_FP32) k_fd_kinetic<float><<<grid, kFdThreads, 0, st>>>((const float2 *) psi, a, partial);
   else k_fd_kinetic<double><<<grid, kFdThreads, 0, st>>>((const double2 *) psi, a, partial);
   GB_CHECK_LAUNCH("fd kinetic");
   k_finish_fd<<<1, 256, 0, st>>>(partial, nb, res);
