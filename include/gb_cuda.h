@@ -83,9 +83,11 @@ long gb_launch_count(void);
  * captures the library stream, so the kernels the following calls issue are
  * recorded instead of run; gb_graph_end instantiates them (*graph receives a
  * handle); gb_graph_launch replays them on the library stream with the same
- * arguments and pointers; gb_graph_free releases the handle.  Captured calls
- * must not read results back to the host; run the same calls once without
- * capture first, so that scratch buffers already have their size. */
+ * arguments and pointers (and with tables of its own, so calls between the
+ * replays may have other parameters); gb_graph_free releases the handle.
+ * Captured calls must not read results back to the host; run the same calls
+ * once without capture first, so that scratch buffers already have their
+ * size. */
 int gb_graph_begin(void);
 int gb_graph_end(void **graph);
 int gb_graph_launch(void *graph);

@@ -1013,41 +1013,38 @@ static long pow2_at_most(long v) {
 // Per-axis table cache: rebuilt and uploaded only when (n, bc, cp, c2)
 // change, so a run of identical steps issues no host transfers.
 struct CnCacheEntry {
-  bool valid;
+  int gen;  // gb__table_gen() of the tables, 0: none
+  double2 *tab;
   long n;
   int bc, nseg;
   cd cp, c2;
   FastTables ft;
 };
 static CnCacheEntry g_cn_cache[3];
-static void *g_cn_tab_base = nullptr;
 
 constexpr long kFastMaxN = 4096;  // longest line of the fast path
 
-static double2 *fast_tables(int slot, long n, int bc, cd cp, cd c2, int nseg, cudaStream_t st, CnAxis *a) {
+static double2 *fast_tables(int slot, long n, int bc, cd cp, cd c2, int nseg, CnAxis *a) {
   const long nmax = kFastMaxN;
   if (n > nmax) {
     gb__set_error(1013, "cn: line length above 4096");
     return nullptr;
   }
-  const long per = 6 * nmax + 2 * 5 * 32;
-  double2 *base = (double2 *) gb__scratch(GB_SCR_CN, sizeof(double2) * (size_t) per * 3);
-  if (!base) return nullptr;
-  if (base != g_cn_tab_base) {
-    for (int i = 0; i < 3; i++) g_cn_cache[i].valid = false;
-    g_cn_tab_base = base;
-  }
-  double2 *tab = base + (size_t) per * slot;
   CnCacheEntry &e = g_cn_cache[slot];
-  if (!(e.valid && e.n == n && e.bc == bc && e.nseg == nseg && e.cp == cp && e.c2 == c2)) {
+  if (!(e.gen == gb__table_gen() && e.n == n && e.bc == bc && e.nseg == nseg && e.cp == cp && e.c2 == c2)) {
+    const size_t per = sizeof(double2) * (size_t) (6 * nmax + 2 * 5 * 32);
+    cudaStream_t st;
+    e.gen = 0;
+    e.tab = (double2 *) gb__table_alloc(GB_SCR_CN0 + slot, per, &st);
+    if (!e.tab) return nullptr;
     build_fast_tables(n, bc, cp, c2, nseg, e.ft);
-    if (cudaMemcpyAsync(tab, e.ft.tab.data(), sizeof(double2) * e.ft.tab.size(), cudaMemcpyHostToDevice, st) !=
+    if (cudaMemcpyAsync(e.tab, e.ft.tab.data(), sizeof(double2) * e.ft.tab.size(), cudaMemcpyHostToDevice, st) !=
             cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
       gb__set_error(3, "cn tables h2d");
       return nullptr;
     }
-    e.valid = true;
+    e.gen = gb__table_gen();
     e.n = n;
     e.bc = bc;
     e.nseg = nseg;
@@ -1062,13 +1059,14 @@ static double2 *fast_tables(int slot, long n, int bc, cd cp, cd c2, int nseg, cu
   a->mc = e.ft.mc;
   a->rbc = e.ft.rbc;
   a->qc = e.ft.qc;
-  return tab;
+  return e.tab;
 }
 
 // Tables of a rotating frame's sweep, built on the device when the parameters
 // change (one kernel of a thread per matrix).
 struct CnClassKey {
-  double2 *base;
+  int gen;  // gb__table_gen() of the tables, 0: none
+  double2 *tab;
   long n, ncls;
   int bc;
   cd cp, c2, c3;
@@ -1076,25 +1074,20 @@ struct CnClassKey {
 };
 static CnClassKey g_cls_key[2];
 
-static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off,
-                             cudaStream_t st) {
-  double2 *tab = (double2 *) gb__scratch(axis == 0 ? GB_SCR_CNROT0 : GB_SCR_CNROT1,
-                                         sizeof(double2) * (size_t) (cls_pitch(n) * ncls));
-  if (!tab) return nullptr;
+static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off) {
   CnClassKey &k = g_cls_key[axis];
-  if (k.base == tab && k.n == n && k.ncls == ncls && k.bc == bc && k.cp == cp && k.c2 == c2 && k.c3 == c3 &&
+  if (k.gen == gb__table_gen() && k.n == n && k.ncls == ncls && k.bc == bc && k.cp == cp && k.c2 == c2 && k.c3 == c3 &&
       k.step == step && k.off == off)
-    return tab;
+    return k.tab;
+  cudaStream_t st;
+  k.gen = 0;
+  double2 *tab = (double2 *) gb__table_alloc(axis == 0 ? GB_SCR_CNROT0 : GB_SCR_CNROT1,
+                                             sizeof(double2) * (size_t) (cls_pitch(n) * ncls), &st);
+  if (!tab) return nullptr;
   auto v2 = [](cd z) { return make_double2(z.real(), z.imag()); };
   k_cn_class_tables<<<(unsigned) ((ncls + 31) / 32), 32, 0, st>>>(tab, n, ncls, bc, v2(cp), v2(c2), v2(c3), step, off);
-  gb__count_launch();
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaGetLastError() != cudaSuccess || cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
-    gb__set_error(3, "cn class tables");
-    return nullptr;
-  }
-  // a captured kernel has not run: the tables count as built only by one that has
-  k = cap == cudaStreamCaptureStatusNone ? CnClassKey{tab, n, ncls, bc, cp, c2, c3, step, off} : CnClassKey{};
+  if (gb__table_built(st, "cn class tables")) return nullptr;
+  k = CnClassKey{gb__table_gen(), tab, n, ncls, bc, cp, c2, c3, step, off};
   return tab;
 }
 
@@ -1274,23 +1267,24 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
 
     // in a rotating frame the matrix of an x (y) line depends on its y (x)
     const bool cls = c3 != cd(0.0);
-    // a rotating frame goes on to the general path where the tiles or the
-    // tables (up to 1 GB) of the fast one end; without rotation those are errors
+    // a rotating frame goes on to the general path, which keeps no tables,
+    // where the tiles or the tables (up to 1 GB) of the fast one end and in a
+    // capture whose graph cannot hold tables; without rotation those are errors
     const long ncls = axis == 0 ? g->ny : g->nx;
     const bool fast = !p->absorb && (p->omega == 0.0 || (a.n <= kFastMaxN && (contig || a.outer <= 65535) &&
-                                                         (!cls || cls_pitch(a.n) * ncls <= (1L << 26))));
+                                                         (!cls || cls_pitch(a.n) * ncls <= (1L << 26)) &&
+                                                         !gb__foreign_capture()));
     if (fast && !cls && a.n <= 32 * kLaneSegMax && g_cn_warp_on) {
       const cd cp = c / tstep;
-      double2 *tab = fast_tables(s, a.n, p->boundary, cp, c2, 32, st, &a);
+      double2 *tab = fast_tables(s, a.n, p->boundary, cp, c2, 32, &a);
       if (!tab) return gb_last_error();
       a.tab = tab;
       a.cp = make_double2(cp.real(), cp.imag());
       GB_TRYC(launch_cn_warp(psi, a, contig, axis, st));
     } else if (fast) {
       const cd cp = c / tstep;
-      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step,
-                                        a.coord_off, st)
-                         : fast_tables(s, a.n, p->boundary, cp, c2, kSeg, st, &a);
+      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step, a.coord_off)
+                         : fast_tables(s, a.n, p->boundary, cp, c2, kSeg, &a);
       if (!tab) return gb_last_error();
       a.tab = tab;
       a.cp = make_double2(cp.real(), cp.imag());

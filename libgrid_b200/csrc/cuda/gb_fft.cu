@@ -55,13 +55,12 @@ struct KinKey {
   int prec, unshifted;
 };
 static KinKey g_kin_key;
-static bool g_kin_valid = false;
+static int g_kin_gen = 0;  // gb__table_gen() of the kept tables
+static unsigned char *g_kin_base = nullptr;
 
 int gb__kin_tables(const gb_geom *g, const gb_kinetic *kin, int unshifted, GbKinTables *out) {
   const long tot = g->nx + g->ny + g->nz;
   const size_t facb = (size_t) tot * 16, sqb = (size_t) tot * 8;
-  unsigned char *base = (unsigned char *) gb__scratch(GB_SCR_KIN, facb + sqb);
-  if (!base) return gb_last_error();
   KinKey key;
   memset(&key, 0, sizeof(key));
   key.nx = g->nx;
@@ -75,23 +74,30 @@ int gb__kin_tables(const gb_geom *g, const gb_kinetic *kin, int unshifted, GbKin
   key.kz0 = unshifted ? 0.0 : kin->kz0;
   key.prec = g->prec;
   key.unshifted = unshifted;
-  double *ksq = (double *) (base + facb);
   const size_t esz = (g->prec == GB_FP32) ? 8 : 16;
-  if (!g_kin_valid || memcmp(&key, &g_kin_key, sizeof(key)) != 0) {
+  if (g_kin_gen != gb__table_gen() || memcmp(&key, &g_kin_key, sizeof(key)) != 0) {
+    cudaStream_t st;
+    g_kin_gen = 0;
+    unsigned char *base = (unsigned char *) gb__table_alloc(GB_SCR_KIN, facb + sqb, &st);
+    if (!base) return gb_last_error();
+    double *ksq = (double *) (base + facb);
     const double lx = 2.0 * M_PI / (g->step * (double) g->nx);
     const double ly = 2.0 * M_PI / (g->step * (double) g->ny);
     const double lz = 2.0 * M_PI / (g->step * (double) g->nz);
     const unsigned nb = (unsigned) ((tot + 255) / 256);
     if (g->prec == GB_FP32)
-      k_kin_tables<float><<<nb, 256, 0, gb__stream()>>>((float2 *) base, ksq, g->nx, g->ny, g->nz, lx, ly, lz,
-                                                         key.kx0, key.ky0, key.kz0, key.tm_re, key.tm_im);
+      k_kin_tables<float><<<nb, 256, 0, st>>>((float2 *) base, ksq, g->nx, g->ny, g->nz, lx, ly, lz, key.kx0, key.ky0,
+                                              key.kz0, key.tm_re, key.tm_im);
     else
-      k_kin_tables<double><<<nb, 256, 0, gb__stream()>>>((double2 *) base, ksq, g->nx, g->ny, g->nz, lx, ly, lz,
-                                                          key.kx0, key.ky0, key.kz0, key.tm_re, key.tm_im);
-    GB_CHECK_LAUNCH("kinetic tables");
+      k_kin_tables<double><<<nb, 256, 0, st>>>((double2 *) base, ksq, g->nx, g->ny, g->nz, lx, ly, lz, key.kx0, key.ky0,
+                                               key.kz0, key.tm_re, key.tm_im);
+    if (gb__table_built(st, "kinetic tables")) return gb_last_error();
     g_kin_key = key;
-    g_kin_valid = true;
+    g_kin_base = base;
+    g_kin_gen = gb__table_gen();
   }
+  unsigned char *base = g_kin_base;
+  double *ksq = (double *) (base + facb);
   out->kfac[0] = base;
   out->kfac[1] = base + esz * (size_t) g->nx;
   out->kfac[2] = base + esz * (size_t) (g->nx + g->ny);

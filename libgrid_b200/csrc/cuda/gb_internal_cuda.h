@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_runtime.h>
 #include <stddef.h>
 
 #include "gb_cuda.h"
@@ -11,19 +12,31 @@ enum {
   GB_SCR_KIN = 0,      // kinetic factor tables
   GB_SCR_PARTIAL = 1,  // reduction partial sums
   GB_SCR_RESULT = 2,   // final reduction results
-  GB_SCR_CN = 3,       // line-solver coefficient tables
+  GB_SCR_NORM = 3,     // renormalisation factor, counter and partial sums of the relaxation steps
   GB_SCR_WORK = 4,     // temporary full grids
   GB_SCR_STAGE = 5,    // precision-conversion staging
   GB_SCR_KIN2 = 6,     // kinetic factor tables of the merged K(dt) pass
   GB_SCR_CHAIN = 7,    // tile counters and ticket of the plane-chained passes
   GB_SCR_UNET = 8,     // per-chunk weight-gradient partials of the U-Net kernels
-  GB_SCR_NORM = 9,     // renormalisation factor, counter and partial sums of the relaxation steps
-  GB_SCR_CNROT0 = 10,  // line-solver tables of a rotating frame's x sweep
-  GB_SCR_CNROT1 = 11,  // and of its y sweep
-  GB_SCR_COUNT = 12
+  GB_SCR_CN0 = 9,      // line-solver coefficient tables of the first sweep; 10 and 11: of the second and third
+  GB_SCR_CNROT0 = 12,  // line-solver tables of a rotating frame's x sweep
+  GB_SCR_CNROT1 = 13,  // and of its y sweep
+  GB_SCR_COUNT = 14
 };
 
 void *gb__scratch(int slot, size_t bytes);
+// Tables kept from call to call under a key of the call's parameters.  A kept
+// table counts while gb__table_gen() is what it was when the table was built
+// (it changes at gb_shutdown and where gb_graph_begin's capture starts and
+// ends).  gb__table_alloc gives the memory for a new one, the scratch slot or,
+// in a capture, memory of the graph, and the stream its building kernel goes
+// to; gb__table_built follows that launch.
+int gb__table_gen(void);
+void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st);
+int gb__table_built(cudaStream_t st, const char *where);
+// Whether the library stream is being captured by other means than
+// gb_graph_begin (the library then owns no memory of the graph).
+bool gb__foreign_capture(void);
 // Pass timing brackets (no-ops unless gb_pass_timing(1) was called).
 int gb__pass_begin(int kind);
 void gb__pass_end(int slot);

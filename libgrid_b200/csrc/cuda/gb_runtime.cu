@@ -12,6 +12,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <new>
+#include <vector>
+
 #include <cudaTypedefs.h>
 
 #include "gb_common.cuh"
@@ -34,6 +37,18 @@ static void free_retired(void) {
   for (int i = 0; i < g_nretired; i++) cudaFree(g_retired[i]);
   g_nretired = 0;
 }
+
+// Tables keyed by a call's parameters (kinetic factors, line-solver
+// coefficients) are kept from call to call, each with its key at the code that
+// builds it.  A key counts only under the generation it was written in.
+static int g_table_gen = 1;
+// While gb_graph_begin records, tables live in memory of the graph: a replay
+// reads them whatever other calls have put into the scratch slots since.
+// They are written at once on a stream beside the captured one, so a replay
+// finds them ready and a plain call never sees them.
+static bool g_capturing = false;
+static std::vector<void *> g_capture_tables;
+static cudaStream_t g_table_stream = nullptr;
 
 static cudaEvent_t g_events[16];
 static bool g_events_made = false;
@@ -89,6 +104,7 @@ extern "C" int gb_init(int device) {
 extern "C" int gb_shutdown(void) {
   if (!g_stream) return 0;
   cudaStreamSynchronize(g_stream);
+  g_table_gen++;
   for (int i = 0; i < GB_SCR_COUNT; i++) {
     if (g_scratch[i].p) cudaFree(g_scratch[i].p);
     g_scratch[i].p = nullptr;
@@ -129,23 +145,38 @@ extern "C" long gb_launch_count(void) { return g_launches; }
 // stream, so the kernels and copies the following calls issue are recorded
 // instead of run; gb_graph_end instantiates them into an executable graph
 // that gb_graph_launch replays on the stream (the same kernels with the same
-// arguments and pointers).  Calls that read results back to the host must
-// not be captured; scratch buffers are best sized by one uncaptured run of
-// the same calls first (a capture must not free device memory).
+// arguments and pointers).  Tables of the captured calls belong to the graph.
+// Calls that read results back to the host must not be captured; scratch
+// buffers are best sized by one uncaptured run of the same calls first (a
+// capture must not free device memory).
 struct GbGraph {
   cudaGraphExec_t exec;
   long kernels;  // launches recorded, added to gb_launch_count per replay
+  std::vector<void *> tables;
 };
 static long g_capture_start = 0;
 
+static void free_tables(std::vector<void *> &t) {
+  if (!t.empty()) cudaStreamSynchronize(g_stream);
+  for (void *p : t) cudaFree(p);
+  t.clear();
+}
+
 extern "C" int gb_graph_begin(void) {
   if (!g_stream) return gb__set_error(1080, "graph: library not initialised");
+  if (!g_table_stream && cudaStreamCreateWithFlags(&g_table_stream, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    g_table_stream = nullptr;
+    return gb__set_error(2, "graph: table stream");
+  }
   const cudaError_t e = cudaStreamBeginCapture(g_stream, cudaStreamCaptureModeRelaxed);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return gb__set_error((int) e, "graph: begin capture");
   }
   g_capture_start = g_launches;
+  g_capturing = true;
+  g_table_gen++;
   return 0;
 }
 
@@ -155,9 +186,14 @@ extern "C" int gb_graph_end(void **out) {
   const cudaError_t e = cudaStreamEndCapture(g_stream, &gr);
   const long kernels = g_launches - g_capture_start;
   g_launches = g_capture_start;
+  if (g_capturing) g_table_gen++;
+  g_capturing = false;
+  std::vector<void *> tables;
+  tables.swap(g_capture_tables);
   if (e != cudaSuccess || !gr) {
     if (gr) cudaGraphDestroy(gr);
     cudaGetLastError();
+    free_tables(tables);
     return gb__set_error(e != cudaSuccess ? (int) e : 1081, "graph: end capture");
   }
   cudaGraphExec_t ex = nullptr;
@@ -165,15 +201,18 @@ extern "C" int gb_graph_end(void **out) {
   cudaGraphDestroy(gr);
   if (ei != cudaSuccess) {
     cudaGetLastError();
+    free_tables(tables);
     return gb__set_error((int) ei, "graph: instantiate");
   }
-  GbGraph *g = (GbGraph *) malloc(sizeof(GbGraph));
+  GbGraph *g = new (std::nothrow) GbGraph;
   if (!g) {
     cudaGraphExecDestroy(ex);
+    free_tables(tables);
     return gb__set_error(2, "graph: host allocation");
   }
   g->exec = ex;
   g->kernels = kernels;
+  g->tables.swap(tables);
   g_graphs_live++;
   *out = g;
   return 0;
@@ -192,7 +231,8 @@ extern "C" int gb_graph_free(void *h) {
   GbGraph *g = (GbGraph *) h;
   if (g) {
     cudaGraphExecDestroy(g->exec);
-    free(g);
+    free_tables(g->tables);
+    delete g;
     if (--g_graphs_live == 0) free_retired();
   }
   return 0;
@@ -302,6 +342,39 @@ void *gb__scratch(int slot, size_t bytes) {
   }
   s.bytes = want;
   return s.p;
+}
+
+int gb__table_gen(void) { return g_table_gen; }
+
+// Memory for a table about to be built, and the stream to build it on.
+void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st) {
+  *st = g_stream;
+  if (!g_capturing) return gb__scratch(slot, bytes);
+  *st = g_table_stream;
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    gb__set_error(2, "graph: table cudaMalloc");
+    return nullptr;
+  }
+  g_capture_tables.push_back(p);
+  return p;
+}
+
+// After the kernel that builds a table was launched on *st: on the library
+// stream the kernels that read the table come after it, a graph's table is
+// waited for.
+int gb__table_built(cudaStream_t st, const char *where) {
+  cudaError_t e = cudaGetLastError();
+  if (st == g_stream) gb__count_launch();
+  else if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  return e == cudaSuccess ? 0 : gb__set_error((int) e, where);
+}
+
+// The library stream is being captured, but not by gb_graph_begin.
+bool gb__foreign_capture(void) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return !g_capturing && cudaStreamIsCapturing(g_stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
 }
 
 // ------------------------------------------------------------ pass timing

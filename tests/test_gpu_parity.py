@@ -287,6 +287,28 @@ def test_cn_rotation(b200, restate, bc, shape):
 
 
 @pytest.mark.parametrize("bc", [DIR, NEU, PER])
+@pytest.mark.parametrize("shape", [(16, 12, 10), (33, 70, 7), (20, 41, 1)])
+def test_cn_rotation_changing(b200, restate, bc, shape):
+    """Time step, rotation and momentum that change from step to step: every
+    sweep's tables are rebuilt right before it."""
+    step, mass = 0.3, 1.0
+    rng = np.random.default_rng(37)
+    psi0 = smooth_state(shape, step) + 0.01 * rand_c(rng, shape)
+    v = 0.02 * rng.standard_normal(shape).astype(complex)
+    w = b200.wf(*shape, step, mass, bc, CN2, values=psi0)
+    pot = b200.cgrid(*shape, step, values=v)
+    want = psi0.copy()
+    for time, omega, k0 in ((0.05, 0.3, 0.0), (0.025, 0.3, 0.0), (0.05, -0.2, 0.1), (0.05, 0.0, 0.1), (0.05, 0.3, 0.0)) * 2:
+        b200.lib.cgrid_set_rotation(w.s.grid, omega)
+        b200.lib.cgrid_set_momentum(w.s.grid, k0, -k0, k0)
+        w.propagate(pot, time)
+        want = restate.cn_step(want, step, mass, time, bc, k0=(k0, -k0, k0), omega=omega, vc=v)
+    assert rel(w.grid.get(), want) < TOL_PSI
+    b200.free(w)
+    b200.free(pot)
+
+
+@pytest.mark.parametrize("bc", [DIR, NEU, PER])
 @pytest.mark.parametrize("shape", [(16, 192, 200), (256, 4, 33)])
 def test_cn_line_solvers_agree(b200, bc, shape):
     """The warp-cooperative line solver (lines up to 256 points, segment
