@@ -170,8 +170,8 @@ __device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int 
         // streaming loads: V is read once per sweep, and evict-first keeps
         // the solver's coefficient tables in the small L1 left beside the
         // shared-memory tiles
-        if (pt.kind == GB_POT_COMPLEX) v[k] = __ldcs((const double2 *) pt.v + vi);
-        else if (pt.kind == GB_POT_REAL) v[k].x = __ldcs((const double *) pt.v + vi);
+        if (pt.kind == GB_POT_COMPLEX) v[k] = ld_cs((const double2 *) pt.v + vi);
+        else if (pt.kind == GB_POT_REAL) v[k].x = ld_cs((const double *) pt.v + vi);
       }
     }
 #pragma unroll
@@ -1074,8 +1074,10 @@ struct CnClassKey {
 };
 static CnClassKey g_cls_key[2];
 
-static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off) {
+static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off,
+                             bool *built) {
   CnClassKey &k = g_cls_key[axis];
+  *built = false;
   if (k.gen == gb__table_gen() && k.n == n && k.ncls == ncls && k.bc == bc && k.cp == cp && k.c2 == c2 && k.c3 == c3 &&
       k.step == step && k.off == off)
     return k.tab;
@@ -1087,6 +1089,7 @@ static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, 
   auto v2 = [](cd z) { return make_double2(z.real(), z.imag()); };
   k_cn_class_tables<<<(unsigned) ((ncls + 31) / 32), 32, 0, st>>>(tab, n, ncls, bc, v2(cp), v2(c2), v2(c3), step, off);
   if (gb__table_built(st, "cn class tables")) return nullptr;
+  *built = true;
   k = CnClassKey{gb__table_gen(), tab, n, ncls, bc, cp, c2, c3, step, off};
   return tab;
 }
@@ -1178,9 +1181,10 @@ template <bool CONTIG, bool CLS> static FastKernel fast_kernel(long n) {
 // Sweeps of up to two waves (two CTAs on each of 148 SMs) overlap the end of
 // the one before: 100 x 100 x 50 in a rotating frame 70.8 -> 66.6 us a step,
 // 125 x 99 x 75 82.9 -> 81.9 us.  With more waves the waiting CTAs only take
-// slots: 192^3 (four waves) 341.1 -> 343.2 us.
-static void cn_launch(FastKernel kern, dim3 grid, size_t smem, cudaStream_t st, void *psi, const CnAxis &a) {
-  if ((long) grid.x * grid.y <= 2 * 296) launch_overlapped(kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
+// slots: 192^3 (four waves) 341.1 -> 343.2 us.  A sweep right after the kernel
+// that built its tables does not overlap it: the tables are read as constants.
+static void cn_launch(FastKernel kern, dim3 grid, size_t smem, cudaStream_t st, void *psi, const CnAxis &a, bool built) {
+  if (!built && (long) grid.x * grid.y <= 2 * 296) launch_overlapped(kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
   else kern<<<grid, 32 * kSeg, smem, st>>>((double2 *) psi, a);
 }
 
@@ -1283,7 +1287,8 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
       GB_TRYC(launch_cn_warp(psi, a, contig, axis, st));
     } else if (fast) {
       const cd cp = c / tstep;
-      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step, a.coord_off)
+      bool built = false;
+      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step, a.coord_off, &built)
                          : fast_tables(s, a.n, p->boundary, cp, c2, kSeg, &a);
       if (!tab) return gb_last_error();
       a.tab = tab;
@@ -1314,7 +1319,7 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         const long nb = (a.outer + lpc - 1) / lpc;
         {
           const int slot = gb__pass_begin(15 + axis);
-          cn_launch(kern, dim3((unsigned) nb), sm, st, psi, a);
+          cn_launch(kern, dim3((unsigned) nb), sm, st, psi, a, built);
           gb__pass_end(slot);
         }
       } else {
@@ -1333,7 +1338,7 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         dim3 grid((unsigned) ((a.inner + lpc - 1) / lpc), (unsigned) a.outer);
         {
           const int slot = gb__pass_begin(15 + axis);
-          cn_launch(kern, grid, sm, st, psi, a);
+          cn_launch(kern, grid, sm, st, psi, a, built);
           gb__pass_end(slot);
         }
       }

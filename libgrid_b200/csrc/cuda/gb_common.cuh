@@ -178,17 +178,39 @@ extern "C" cudaStream_t gb__stream(void);
 // ------------------------------------------------------------------------
 // Launches whose start overlaps the end of the kernel before them on the
 // stream (programmatic dependent launch).  Every CTA of such a kernel calls
-// grid_wait on each pointer it reads before it touches global memory: it
-// returns when the kernels before have finished and their writes are visible.
-// The pointer passes through the statement, so that no load of it, a read-only
-// one of a restrict pointer included, can be moved above.  The next launch is
-// let go right after, when all CTAs of this one have started.  For the line
-// passes, launch by launch / overlapped: a 32^3 step (nine passes) 38.9 / 23.2
-// us, a 128^3 convolution 135 / 117 us, ten relaxation steps at 128^3 909 / 822
-// us, a 256^3 step 888 / 889 us (FP64).
+// grid_wait before it touches global memory: it returns when the kernels before
+// have finished and their writes are visible.  The next launch is let go right
+// after, when all CTAs of this one have started.  The compiler must not move a
+// load above the statement:
+// - what a restrict pointer reads (as read-only loads) goes through the pointer
+//   that grid_wait was given;
+// - plain loads of other pointers, cp.async and bulk copies stay below it;
+// - the cache-hint intrinsics (__ldcg, __ldcs) are not known to: ld_cg and
+//   ld_cs take their place;
+// - __ldg is for what no kernel can still be writing: tables are written by a
+//   kernel whose next one on the stream was launched without overlap.
+// For the line passes, launch by launch / overlapped: a 32^3 step (nine passes)
+// 38.9 / 23.2 us, a 128^3 convolution 135 / 117 us, ten relaxation steps at
+// 128^3 909 / 822 us, a 256^3 step 888 / 889 us (FP64).
 template <typename P> __device__ __forceinline__ void grid_wait(P &p) {
   asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ double ld_cg(const double *p) {
+  double v;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_cs(const double *p) {
+  double v;
+  asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_cs(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
 }
 
 template <typename... Params, typename... Args>

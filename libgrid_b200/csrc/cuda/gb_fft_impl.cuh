@@ -472,7 +472,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
     } else if constexpr (Op == OP_INV) {
       fft_line<T2, +1, N>(v, t, sm, tw);
     } else if constexpr (Op == OP_SCALE) {
-      const T s = (T) (a.pscale ? a.scale * __ldcg(a.pscale) : a.scale);
+      const T s = (T) (a.pscale ? a.scale * ld_cg(a.pscale) : a.scale);
 #pragma unroll
       for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
     } else if constexpr (Op == OP_KIN || Op == OP_KIN2) {
@@ -523,7 +523,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
       pot_row(a, o, q, i0, j0, k0, vbase, vstride);
       const gb_potential &pt = a.pot;
       if (a.pscale) {  // psi renormalised first
-        const T s = (T) __ldcg(a.pscale);
+        const T s = (T) ld_cg(a.pscale);
 #pragma unroll
         for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
       }
@@ -610,7 +610,7 @@ template <int THREADS> __device__ __forceinline__ double block_sum(double v, dou
 }
 
 // Sum of the blocks' OP_KIN2 sums: every block leaves its partial, and the
-// last one to finish adds them in block order and writes the renormalisation
+// last one to finish adds them in a fixed order and writes the renormalisation
 // factor, so the result does not depend on which block that is and no further
 // launch is needed.  The counter wraps back to 0.
 template <int THREADS>
@@ -640,7 +640,7 @@ __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsig
   if (!s_last) return;
   __threadfence();
   double s = 0.0;
-  for (unsigned i = threadIdx.x; i < nblk; i += THREADS) s += __ldcg(a.partial + i);
+  for (unsigned i = threadIdx.x; i < nblk; i += THREADS) s += ld_cg(a.partial + i);
   r = sum(s);
   if (threadIdx.x == 0) {
     const double nrm = r * a.nfactor;
