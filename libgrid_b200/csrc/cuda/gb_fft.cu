@@ -143,6 +143,23 @@ int gb__sum_partials(const double *partial, long n, double *out_host) {
   return gb__read_result(out_host, sizeof(double));
 }
 
+// The renormalisation factor from the partial sums of a pass of many blocks.
+__global__ void __launch_bounds__(1024) k_norm_finish(const double *p, long n, double target, double factor, double *out) {
+  __shared__ double sbuf[32];
+  grid_wait(p);
+  double s = 0.0;
+#pragma unroll 8
+  for (long i = threadIdx.x; i < n; i += 1024) s += ld_cg(p + i);
+  const double nrm = gbfft::block_sum<1024>(s, sbuf) * factor;
+  if (threadIdx.x == 0) *out = nrm > 0.0 ? sqrt(target / nrm) : 1.0;
+}
+
+int gb__norm_finish(const double *partial, long n, double target, double factor, double *out) {
+  launch_overlapped(k_norm_finish, dim3(1), 1024, 0, gb__stream(), partial, n, target, factor, out);
+  GB_CHECK_LAUNCH("renormalisation");
+  return 0;
+}
+
 // ------------------------------------------------- standalone pointwise ops
 
 // psi_k *= exp(tm |k - k0|^2) (zero beyond the cutoff), evaluated per point

@@ -29,6 +29,9 @@
 // Tensor maps for the pipelined strided passes and their error flag
 // (gb_runtime.cu).
 int gb__tmap_lines(CUtensorMap *out, const void *base, long outer, long n, long inner, int fp32, int bz, int rows);
+// *out = sqrt(target / (factor * sum of the n partial sums)), 1 for a sum that
+// is not positive (gb_fft.cu).
+int gb__norm_finish(const double *partial, long n, double target, double factor, double *out);
 
 namespace gbfft {
 
@@ -612,25 +615,26 @@ template <int THREADS> __device__ __forceinline__ double block_sum(double v, dou
 // Sum of the blocks' OP_KIN2 sums: every block leaves its partial, and the
 // last one to finish adds them in a fixed order and writes the renormalisation
 // factor, so the result does not depend on which block that is and no further
-// launch is needed.  The counter wraps back to 0.
+// launch is needed.  The counter wraps back to 0.  Without a counter the sum is
+// left to gb__norm_finish (norm_in_pass).
 template <int THREADS>
 __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsigned blk, unsigned nblk) {
-  __shared__ double sbuf[THREADS % 32 ? THREADS : THREADS / 32];
+  __shared__ double sbuf[THREADS / 32 + 1];
   __shared__ bool s_last;
-  // blocks of less than a warp (short lines, single columns) sum in order
   auto sum = [&](double v) -> double {
-    if constexpr (THREADS % 32) {
-      sbuf[threadIdx.x] = v;
-      __syncthreads();
-      double t = 0.0;
-      if (threadIdx.x == 0)
-        for (int i = 0; i < THREADS; i++) t += sbuf[i];
-      return t;
+    if constexpr (THREADS < 32) {  // short lines, single columns: part of a warp
+#pragma unroll
+      for (int off = THREADS / 2; off > 0; off /= 2) v += __shfl_down_sync((1u << THREADS) - 1u, v, off);
+      return v;
     } else {
       return block_sum<THREADS>(v, sbuf);
     }
   };
   double r = sum(acc);
+  if (!a.ndone) {
+    if (threadIdx.x == 0) a.partial[blk] = r;
+    return;
+  }
   if (threadIdx.x == 0) {
     a.partial[blk] = r;
     __threadfence();
@@ -647,6 +651,16 @@ __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsig
     *a.sout = nrm > 0.0 ? sqrt(a.ntarget / nrm) : 1.0;
   }
 }
+
+// Whether the last block of a renormalising pass adds the partial sums.  Every
+// block then waits for its sum to be visible and for a shared counter, and the
+// last one, of as few as eight threads (lines of up to 16 points), is alone on
+// the chip; more blocks than a few per SM are faster with a launch of their own
+// for the sum.  Ten relaxation steps, in the pass / by a launch, FP64, us: 32^3
+// (128 blocks) 145 / 146 and FP32 130 / 138; 512 x 64 x 64 (512 blocks of 256
+// threads) 702 / 694; 512 x 128 x 128 (2048) 3460 / 3300; 16 x 128 x 128 (2048
+// blocks of 8) 440 / 280; 16 x 512 x 512 (32768) 4760 / 1850.
+inline bool norm_in_pass(long nblk) { return nblk <= 256; }
 
 // ---------------------------------------------------------------- kernels
 
@@ -887,6 +901,20 @@ int launch_strided_pipe(const void *src, void *dst, const PassArgs &a, long oute
   }
 }
 
+// Arguments of a pass of `grid` blocks: without the counter where the sum of a
+// renormalising pass is a launch of its own (norm_after, once the pass is
+// launched).
+template <int... Ops> PassArgs norm_args(const PassArgs &a, dim3 grid, OpL<Ops...> ops) {
+  PassArgs r = a;
+  if (has_norm(ops) && !norm_in_pass((long) grid.x * grid.y)) r.ndone = nullptr;
+  return r;
+}
+inline int norm_after(const PassArgs &a, dim3 grid) {
+  GB_CHECK_LAUNCH("fft pass");
+  const long n = (long) grid.x * grid.y;
+  return norm_in_pass(n) ? 0 : gb__norm_finish(a.partial, n, a.ntarget, a.nfactor, a.sout);
+}
+
 // Launch one pass of program Ops along `axis` for line length N.
 template <typename T, int N, int... Ops>
 int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, long inner, long *nblocks) {
@@ -898,17 +926,17 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
     if constexpr (has_norm(OpL<Ops...>{})) {  // the outermost of two or more axes is never contiguous
       return gb__set_error(1007, "fft pass: contiguous renormalising pass");
     } else {
-    using Cfg = ContigCfg<N, sizeof(T)>;
-    const size_t sm = (size_t) Cfg::L * Cfg::LINE * sizeof(T2) + STAGE * Cfg::THREADS;
-    auto kern = k_pass_contig<T, N, Ops...>;
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
-      attr_set = true;
-    }
-    const long nb = (outer + Cfg::L - 1) / Cfg::L;
-    if (nblocks) *nblocks = nb;
-    launch_overlapped(kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst, outer, a);
+      using Cfg = ContigCfg<N, sizeof(T)>;
+      const size_t sm = (size_t) Cfg::L * Cfg::LINE * sizeof(T2) + STAGE * Cfg::THREADS;
+      auto kern = k_pass_contig<T, N, Ops...>;
+      static bool attr_set = false;
+      if (!attr_set) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
+        attr_set = true;
+      }
+      const long nb = (outer + Cfg::L - 1) / Cfg::L;
+      if (nblocks) *nblocks = nb;
+      launch_overlapped(kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst, outer, a);
     }
   } else {
     constexpr int BZ = StridedCfg<N, sizeof(T)>::BZ;
@@ -927,7 +955,9 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) (inner / BZ), (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      launch_overlapped(kern, grid, (N / Sched<N>::P) * BZ, sm, st, (const T2 *) src, (T2 *) dst, inner, a);
+      launch_overlapped(kern, grid, (N / Sched<N>::P) * BZ, sm, st, (const T2 *) src, (T2 *) dst, inner,
+                        norm_args(a, grid, OpL<Ops...>{}));
+      if constexpr (has_norm(OpL<Ops...>{})) return norm_after(a, grid);
     } else if (outer <= 65535) {
       const size_t sm = (size_t) N * sizeof(T2) + STAGE * (N / Sched<N>::P);
       auto kern = k_pass_strided<T, N, 1, Ops...>;
@@ -938,7 +968,9 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) inner, (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      launch_overlapped(kern, grid, N / Sched<N>::P, sm, st, (const T2 *) src, (T2 *) dst, inner, a);
+      launch_overlapped(kern, grid, N / Sched<N>::P, sm, st, (const T2 *) src, (T2 *) dst, inner,
+                        norm_args(a, grid, OpL<Ops...>{}));
+      if constexpr (has_norm(OpL<Ops...>{})) return norm_after(a, grid);
     } else {
       return gb__set_error(1001, "fft pass: outer extent above 65535");
     }
