@@ -1184,8 +1184,8 @@ template <bool CONTIG, bool CLS> static FastKernel fast_kernel(long n) {
 // slots: 192^3 (four waves) 341.1 -> 343.2 us.  A sweep right after the kernel
 // that built its tables does not overlap it: the tables are read as constants.
 static void cn_launch(FastKernel kern, dim3 grid, size_t smem, cudaStream_t st, void *psi, const CnAxis &a, bool built) {
-  if (!built && (long) grid.x * grid.y <= 2 * 296) launch_overlapped(kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
-  else kern<<<grid, 32 * kSeg, smem, st>>>((double2 *) psi, a);
+  const bool overlap = !built && (long) grid.x * grid.y <= 2 * 296;
+  launch_stream(overlap, kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
 }
 
 static int g_cn_warp_on = 0;

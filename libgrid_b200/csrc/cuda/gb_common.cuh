@@ -189,9 +189,9 @@ extern "C" cudaStream_t gb__stream(void);
 //   ld_cs take their place;
 // - __ldg is for what no kernel can still be writing: tables are written by a
 //   kernel whose next one on the stream was launched without overlap.
-// For the line passes, launch by launch / overlapped: a 32^3 step (nine passes)
-// 38.9 / 23.2 us, a 128^3 convolution 135 / 117 us, ten relaxation steps at
-// 128^3 909 / 822 us, a 256^3 step 888 / 889 us (FP64).
+// Which launches overlap: pass_overlaps in gb_fft_impl.cuh, cn_launch in
+// gb_cn.cu.  Launched without overlap (launch_stream with false) such a kernel
+// runs as any other.
 template <typename P> __device__ __forceinline__ void grid_wait(P &p) {
   asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -214,8 +214,8 @@ __device__ __forceinline__ double2 ld_cs(const double2 *p) {
 }
 
 template <typename... Params, typename... Args>
-inline void launch_overlapped(void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
-                              Args... args) {
+inline void launch_stream(bool overlap, void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem,
+                          cudaStream_t st, Args... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -225,7 +225,7 @@ inline void launch_overlapped(void (*kern)(Params...), dim3 grid, unsigned threa
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, Params(args)...);  // the caller checks the launch
 }
 

@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(1024) k_norm_finish(const double *p, long n, d
 }
 
 int gb__norm_finish(const double *partial, long n, double target, double factor, double *out) {
-  launch_overlapped(k_norm_finish, dim3(1), 1024, 0, gb__stream(), partial, n, target, factor, out);
+  launch_stream(true, k_norm_finish, dim3(1), 1024, 0, gb__stream(), partial, n, target, factor, out);
   GB_CHECK_LAUNCH("renormalisation");
   return 0;
 }

@@ -55,3 +55,23 @@ def test_relaxation_steps_beat_single_calls(b200, shape):
     assert _ms(b200.lib, merged) < 0.9 * _ms(b200.lib, single)
     b200.free(w)
     b200.free(v)
+
+
+@pytest.mark.parametrize("shape", [(64, 512, 512), (512, 128, 128), (128, 64, 64)])
+def test_overlapped_passes_beat_passes_apart(b200, shape):
+    """A step whose launches may overlap against the same step with an event
+    between any two of them, which keeps them apart: at most the spread of the
+    least times slower (5%)."""
+    w, v = _fluid(b200, shape)
+
+    def steps():
+        for _ in range(4):
+            w.propagate_gp(v, 1e-3, 1.0)
+
+    steps()
+    b200.lib.gb_pass_timing(1)
+    apart = _ms(b200.lib, steps)
+    b200.lib.gb_pass_timing(0)
+    assert _ms(b200.lib, steps) < 1.05 * apart
+    b200.free(w)
+    b200.free(v)
