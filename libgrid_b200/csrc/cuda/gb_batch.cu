@@ -97,7 +97,7 @@ __device__ __forceinline__ void batch_tile_contig(const BatchInst &I, int tile, 
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
     T *stage = (T *) (smraw + (size_t) L * Cfg::LINE * sizeof(T2)) + threadIdx.x;
-    if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(a, line, 0u, t, stage, THREADS)) vstage = stage;
+    if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(a, line, 0u, t, stage, THREADS)) vstage = stage;
   }
   T2 v[P];
 #pragma unroll
@@ -128,7 +128,7 @@ __device__ __forceinline__ void batch_tile_strided(const BatchInst &I, int tile,
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
     T *stage = (T *) (smraw + (size_t) N * BZ * sizeof(T2)) + threadIdx.x;
-    if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(a, 0u, q, t, stage, THREADS)) vstage = stage;
+    if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(a, 0u, q, t, stage, THREADS)) vstage = stage;
   }
   T2 v[P];
 #pragma unroll

@@ -44,7 +44,7 @@ template <int... Ops> constexpr int prog_id(OpL<Ops...>) {
   if (n == 1 && o[0] == OP_FWD) return 0;
   if (n == 1 && o[0] == OP_INV) return 1;
   if (n == 3 && o[0] == OP_FWD && o[1] == OP_KIN && o[2] == OP_INV) return 2;
-  if (n == 3 && o[0] == OP_INV && o[1] == OP_POT && o[2] == OP_FWD) return 3;
+  if (n == 3 && o[0] == OP_INV && is_pot(o[1]) && o[2] == OP_FWD) return 3;
   return 4;
 }
 
@@ -60,6 +60,12 @@ int pass(const gb_geom *g, int axis, const void *src, void *dst, PassArgs a, OpL
   const int rc = launch_pass<T>(v.n, src, dst, a, v.outer, v.inner, ops);
   gb__pass_end(slot);
   return rc;
+}
+
+// The pass INV.POT.FWD, by the kind of the potential.
+template <typename T> int line_pot_pass(const gb_geom *g, int axis, void *psi, const PassArgs &a) {
+  if (a.pot.kind == GB_POT_COMPLEX && !a.pot.absorb) return pass<T>(g, axis, psi, psi, a, OpL<OP_INV, OP_POT_C, OP_FWD>{});
+  return pass<T>(g, axis, psi, psi, a, OpL<OP_INV, OP_POT_S, OP_FWD>{});
 }
 
 // Plane-chained passes (gb_plane.cuh) for grids whose y and z lines are
@@ -129,7 +135,7 @@ template <typename T> int plane_mid(const gb_geom *g, void *psi, const PassArgs 
     return has_pot ? plane_chain<T>(g, psi, a, 19, Stage<2, OP_INV, OP_POT, OP_FWD>{}, Stage<1, OP_FWD>{})
                    : plane_chain<T>(g, psi, a, 19, Stage<2, OP_INV, OP_FWD>{}, Stage<1, OP_FWD>{});
   } else {
-    rc = has_pot ? pass<T>(g, 2, psi, psi, a, OpL<OP_INV, OP_POT, OP_FWD>{})
+    rc = has_pot ? line_pot_pass<T>(g, 2, psi, a)
                  : pass<T>(g, 2, psi, psi, a, OpL<OP_INV, OP_FWD>{});
     if (!rc) rc = pass<T>(g, 1, psi, psi, a, OpL<OP_FWD>{});
     return rc;
@@ -206,7 +212,7 @@ int gb__split_step_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const g
   GB_TRY((pass<T>(g, last, psi, psi, a, OpL<OP_FWD, OP_KIN, OP_INV>{})));
   for (int s = na - 2; s >= 1; s--) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_INV>{})));
   // innermost axis: back to real space, potential factor, forward again
-  if (has_pot) GB_TRY((pass<T>(g, ax[0], psi, psi, a, OpL<OP_INV, OP_POT, OP_FWD>{})));
+  if (has_pot) GB_TRY(line_pot_pass<T>(g, ax[0], psi, a));
   else GB_TRY((pass<T>(g, ax[0], psi, psi, a, OpL<OP_INV, OP_FWD>{})));
   for (int s = 1; s < na - 1; s++) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_FWD>{})));
   GB_TRY((pass<T>(g, last, psi, psi, a, OpL<OP_FWD, OP_KIN, OP_INV>{})));
@@ -276,7 +282,7 @@ int gb__split_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const 
   for (int st = 0; st < nsteps; st++) {
     GB_TRY((pass<T>(g, last, psi, psi, st == 0 ? ah : af, OpL<OP_FWD, OP_KIN, OP_INV>{})));
     for (int s = na - 2; s >= 1; s--) GB_TRY((pass<T>(g, ax[s], psi, psi, ah, OpL<OP_INV>{})));
-    if (has_pot) GB_TRY((pass<T>(g, ax[0], psi, psi, ah, OpL<OP_INV, OP_POT, OP_FWD>{})));
+    if (has_pot) GB_TRY(line_pot_pass<T>(g, ax[0], psi, ah));
     else GB_TRY((pass<T>(g, ax[0], psi, psi, ah, OpL<OP_INV, OP_FWD>{})));
     for (int s = 1; s < na - 1; s++) GB_TRY((pass<T>(g, ax[s], psi, psi, ah, OpL<OP_FWD>{})));
   }
@@ -341,7 +347,7 @@ int gb__relax_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const 
       GB_TRY(plane_mid<T>(g, psi, ap, true));
     } else {
       for (int s = na - 2; s >= 1; s--) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_INV>{})));
-      GB_TRY((pass<T>(g, ax[0], psi, psi, ap, OpL<OP_INV, OP_POT, OP_FWD>{})));
+      GB_TRY(line_pot_pass<T>(g, ax[0], psi, ap));
       for (int s = 1; s < na - 1; s++) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_FWD>{})));
     }
   }

@@ -38,10 +38,16 @@ namespace gbfft {
 // OP_POT_RP is the potential op for one case only, a real V_ext in real
 // time without an absorbing region (a pure phase), so a kernel built for it
 // carries none of the other potential paths.
+// OP_POT takes every potential; OP_POT_C a complex V without an absorbing region
+// and OP_POT_S all others, each without the registers of the other's path
+// (line_pot_pass chooses).  INV.POT.FWD over 1 x 2048 x 2048 with a real V, with
+// OP_POT / OP_POT_S: FP64 75.8 / 69.7 us, FP32 45.3 / 39.0 us; a 1 x 2048 x 2048
+// step with a complex V in FP32, OP_POT / OP_POT_C: 169 / 158 us.
 // OP_KIN2 is the kinetic factor twice with the sum of |psi|^2 taken between
 // the two (the end of one step and the start of the next, renormalised).
 enum : int {
-  OP_END = 0, OP_FWD = 1, OP_INV = 2, OP_KIN = 3, OP_POT = 4, OP_SCALE = 5, OP_KSQ = 6, OP_POT_RP = 7, OP_KIN2 = 8
+  OP_END = 0, OP_FWD = 1, OP_INV = 2, OP_KIN = 3, OP_POT = 4, OP_SCALE = 5, OP_KSQ = 6, OP_POT_RP = 7, OP_KIN2 = 8,
+  OP_POT_S = 9, OP_POT_C = 10
 };
 
 template <int... Ops> struct OpL {};
@@ -410,11 +416,12 @@ __device__ __forceinline__ bool pot_is_simple(const gb_potential &pt) {
 // thread will need in the potential op into its own shared-memory slots
 // stage[m * stride], m < P, so the load latency overlaps the tile load and
 // the first transform.  Returns false (nothing issued) when the potential
-// op will not read a real V through the simple path.
-template <typename T, int P, int TL, bool ANYPOT>
+// op will not read a real V through the simple path.  POT: the program's
+// potential op.
+template <typename T, int P, int TL, int POT>
 __device__ __forceinline__ bool pot_prefetch(const PassArgs &a, unsigned o, unsigned q, int t, T *stage,
                                              int stride) {
-  const bool cplx = ANYPOT && a.pot.kind == GB_POT_COMPLEX && !a.pot.absorb;
+  const bool cplx = POT == OP_POT_C || (POT == OP_POT && a.pot.kind == GB_POT_COMPLEX && !a.pot.absorb);
   if (!cplx && (a.pot.kind != GB_POT_REAL || !pot_is_simple(a.pot))) return false;
   int i0, j0, k0;
   unsigned vbase, vstride;
@@ -438,11 +445,16 @@ __device__ __forceinline__ bool pot_prefetch(const PassArgs &a, unsigned o, unsi
   return true;
 }
 
-template <int... Ops> __host__ __device__ constexpr bool has_pot(OpL<Ops...>) {
-  return ((Ops == OP_POT || Ops == OP_POT_RP) || ...);
+__host__ __device__ constexpr bool is_pot(int op) {
+  return op == OP_POT || op == OP_POT_S || op == OP_POT_C || op == OP_POT_RP;
 }
-// any potential, not only the one of OP_POT_RP
-template <int... Ops> __host__ __device__ constexpr bool has_anypot(OpL<Ops...>) { return ((Ops == OP_POT) || ...); }
+template <int... Ops> __host__ __device__ constexpr bool has_pot(OpL<Ops...>) { return (is_pot(Ops) || ...); }
+// the potential op of a program that has one
+template <int... Ops> __host__ __device__ constexpr int pot_op(OpL<Ops...>) { return ((is_pot(Ops) ? Ops : 0) + ...); }
+// programs that stage a real V in shared memory
+template <int... Ops> __host__ __device__ constexpr bool has_stage(OpL<Ops...> ops) {
+  return has_pot(ops) && pot_op(ops) != OP_POT_C;
+}
 template <int... Ops> __host__ __device__ constexpr bool has_kin(OpL<Ops...>) {
   return ((Ops == OP_KIN || Ops == OP_KIN2) || ...);
 }
@@ -518,7 +530,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
 #pragma unroll
         for (int m = 0; m < P; m++) v[m] = cmul(v[m], cmul(lf, fa[t + TL * m]));
       }
-    } else if constexpr (Op == OP_POT) {
+    } else if constexpr (Op == OP_POT || Op == OP_POT_S || Op == OP_POT_C) {
       // decode the line once; along the pass axis the potential index
       // advances by a fixed stride
       int i0, j0, k0;
@@ -530,7 +542,9 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
 #pragma unroll
         for (int m = 0; m < P; m++) v[m] = cscale(v[m], s);
       }
-      if (pot_is_simple(pt)) {
+      if constexpr (Op == OP_POT_C) {
+        pot_line_complex<T, P, TL>(v, t, (const T2 *) pt.v + vbase, vstride, pt);
+      } else if (pot_is_simple(pt)) {
         const bool phase = (pt.c_re == 0.0);
         const double cc = phase ? pt.c_im : pt.c_re;
         // V from this thread's prefetched slots when the kernel staged it,
@@ -551,7 +565,7 @@ template <typename T, int N, class SM, int Op, int... Rest> struct Program<T, N,
           if (phase) pot_line_simple<T, P, TL, false, true>(v, t, vp, vt, vm, pt.cons, pt.g, cc);
           else pot_line_simple<T, P, TL, false, false>(v, t, vp, vt, vm, pt.cons, pt.g, cc);
         }
-      } else if (pt.kind == GB_POT_COMPLEX && !pt.absorb) {
+      } else if (Op == OP_POT && pt.kind == GB_POT_COMPLEX && !pt.absorb) {
         pot_line_complex<T, P, TL>(v, t, (const T2 *) pt.v + vbase, vstride, pt);
       } else {
 #pragma unroll
@@ -719,7 +733,7 @@ __global__ void __launch_bounds__(ContigCfg<N, sizeof(T)>::THREADS, ContigCfg<N,
   if constexpr (has_pot(OpL<Ops...>{})) {
     // potential values staged behind the exchange buffer
     T *stage = (T *) (smraw + (size_t) Cfg::L * Cfg::LINE * sizeof(T2)) + threadIdx.x;
-    if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(a, ok ? line : 0u, 0u, t, stage, Cfg::THREADS)) vstage = stage;
+    if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(a, ok ? line : 0u, 0u, t, stage, Cfg::THREADS)) vstage = stage;
   }
   T2 v[P];
 #pragma unroll
@@ -770,7 +784,7 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, pass_min_blocks<(N / S
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
     T *stage = (T *) (smraw + (size_t) N * BZ * sizeof(T2)) + threadIdx.x;
-    if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(a, o, q, t, stage, THREADS)) vstage = stage;
+    if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(a, o, q, t, stage, THREADS)) vstage = stage;
   }
   T2 v[P];
 #pragma unroll
@@ -936,7 +950,7 @@ template <typename T, int N, int... Ops>
 int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, long inner, long *nblocks) {
   using T2 = C2<T>;
   // per-thread staging of the potential values (P reals per thread)
-  constexpr size_t STAGE = has_pot(OpL<Ops...>{}) ? (size_t) Sched<N>::P * sizeof(T) : 0;
+  constexpr size_t STAGE = has_stage(OpL<Ops...>{}) ? (size_t) Sched<N>::P * sizeof(T) : 0;
   cudaStream_t st = gb__stream();
   if (inner == 1) {
     if constexpr (has_norm(OpL<Ops...>{})) {  // the outermost of two or more axes is never contiguous

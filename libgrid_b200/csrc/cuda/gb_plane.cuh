@@ -93,7 +93,7 @@ __device__ __forceinline__ void chain_tile(Stage<AX, Ops...>, C2<T> *__restrict_
     const unsigned line = p * (unsigned) N + tile * (unsigned) W + (unsigned) l;
     const T *vstage = nullptr;
     if constexpr (((Ops == OP_POT || Ops == OP_POT_RP) || ...)) {
-      if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(c.az, line, 0u, t, stage, THREADS)) vstage = stage;
+      if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(c.az, line, 0u, t, stage, THREADS)) vstage = stage;
     }
     T2 *s = psi + (size_t) line * N;
 #pragma unroll
@@ -107,7 +107,7 @@ __device__ __forceinline__ void chain_tile(Stage<AX, Ops...>, C2<T> *__restrict_
     const unsigned q = tile * (unsigned) W + (unsigned) cc;
     const T *vstage = nullptr;
     if constexpr (((Ops == OP_POT || Ops == OP_POT_RP) || ...)) {
-      if (pot_prefetch<T, P, TL, has_anypot(OpL<Ops...>{})>(c.ay, p, q, t, stage, THREADS)) vstage = stage;
+      if (pot_prefetch<T, P, TL, pot_op(OpL<Ops...>{})>(c.ay, p, q, t, stage, THREADS)) vstage = stage;
     }
     T2 *s = psi + (size_t) p * N * N + q;
 #pragma unroll
