@@ -763,7 +763,8 @@ template <int N, int ES = 8> struct StridedCfg {
 };
 
 // Strided lines: block = (column block of BZ adjacent inner indices, outer).
-template <typename T, int N, int BZ, int... Ops>
+// WAIT: may be launched with overlap.
+template <typename T, int N, int BZ, bool WAIT, int... Ops>
 __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, pass_min_blocks<(N / Sched<N>::P) * BZ, sizeof(T)>())
     k_pass_strided(const C2<T> *__restrict__ src, C2<T> *__restrict__ dst, long inner, PassArgs a) {
   using T2 = C2<T>;
@@ -779,7 +780,7 @@ __global__ void __launch_bounds__((N / Sched<N>::P) * BZ, pass_min_blocks<(N / S
   // element (line, t + TL m) sits at base + (t + TL m) * inner; the whole
   // grid has fewer than 2^31 points, so the in-tile offsets fit 32 bits
   const size_t off = (size_t) o * (size_t) N * (size_t) inner + q;
-  grid_wait(src);
+  if constexpr (WAIT) grid_wait(src);
   const T2 *s = src + off;
   const T *vstage = nullptr;
   if constexpr (has_pot(OpL<Ops...>{})) {
@@ -945,6 +946,18 @@ inline int norm_after(const PassArgs &a, dim3 grid) {
   return norm_in_pass(n) ? 0 : gb__norm_finish(a.partial, n, a.ntarget, a.nfactor, a.sout);
 }
 
+// Most CTAs of a pass over lines of N <= 16 points that is launched with
+// overlap.  Such a CTA has 8 or 16 threads and an SM holds 32 of them, so the
+// wait at its start, even one that returns at once, is a large part of its time;
+// more CTAs run in a form without it, after the pass before.  One step, always
+// with the wait / without it beyond the limit, FP64, us: 256 x 4 x 256 (8192
+// CTAs a pass) 62.5 / 52.5; 8 x 256 x 256 (8192) 93.4 / 92.1; 512 x 8 x 256
+// (16384) 119 / 96; 2 x 512 x 512 (32768) 129 / 94; 512 x 4 x 512 (32768) 199 /
+// 136; FP32 512 x 4 x 512 114 / 86.  Below it: 16 x 128 x 128 (2048) 36.1 with,
+// 39.4 without; FP32 4 x 256 x 256 (4096) 46.9, 49.4; of 16 points 16 x 256 x
+// 256 (8192) 108.6, 111.6.
+template <int N> constexpr long kTinyOverlap = N < 16 ? 4096 : 8192;
+
 // Launch one pass of program Ops along `axis` for line length N.
 template <typename T, int N, int... Ops>
 int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, long inner, long *nblocks) {
@@ -977,8 +990,9 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       if (rc || launched) return rc;
     }
     if (inner % BZ == 0 && outer <= 65535) {
-      const size_t sm = (size_t) N * BZ * sizeof(T2) + STAGE * (N / Sched<N>::P) * BZ;
-      auto kern = k_pass_strided<T, N, BZ, Ops...>;
+      constexpr int THREADS = (N / Sched<N>::P) * BZ;
+      const size_t sm = (size_t) N * BZ * sizeof(T2) + STAGE * THREADS;
+      auto kern = k_pass_strided<T, N, BZ, true, Ops...>;
       static bool attr_set = false;
       if (!attr_set) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
@@ -986,12 +1000,19 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) (inner / BZ), (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      launch_stream(pass_overlaps<T>(a), kern, grid, (N / Sched<N>::P) * BZ, sm, st, (const T2 *) src, (T2 *) dst, inner,
+      bool overlap = pass_overlaps<T>(a);
+      if constexpr (THREADS < 32) {
+        if (!overlap || (long) grid.x * grid.y > kTinyOverlap<N>) {
+          overlap = false;
+          kern = k_pass_strided<T, N, BZ, false, Ops...>;
+        }
+      }
+      launch_stream(overlap, kern, grid, THREADS, sm, st, (const T2 *) src, (T2 *) dst, inner,
                     norm_args(a, grid, OpL<Ops...>{}));
       if constexpr (has_norm(OpL<Ops...>{})) return norm_after(a, grid);
     } else if (outer <= 65535) {
       const size_t sm = (size_t) N * sizeof(T2) + STAGE * (N / Sched<N>::P);
-      auto kern = k_pass_strided<T, N, 1, Ops...>;
+      auto kern = k_pass_strided<T, N, 1, true, Ops...>;
       static bool attr_set = false;
       if (!attr_set) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);

@@ -100,6 +100,23 @@ def test_split_step_fft(b200, restate, shape, time):
     assert rel(got, want) < TOL_PSI
 
 
+@pytest.mark.parametrize("prec,tol", [(0, TOL_PSI), (capi.GRID_PREC_FP32, 1e-5)])
+@pytest.mark.parametrize("shape", [(2, 64, 256), (2, 256, 512), (256, 4, 256), (256, 8, 512), (16, 256, 512)])
+def test_split_step_short_axes(b200, restate, shape, prec, tol):
+    """Strided lines of 2 to 16 points, up to and beyond the number of CTAs from
+    which their passes are launched without overlap (FP32: rounding of nine
+    transforms of single precision)."""
+    rng = np.random.default_rng(19)
+    step, mass, time = 0.4, 1.7, 0.05
+    psi0 = rand_c(rng, shape)
+    v = 0.05 * rng.standard_normal(shape) + 0.002j * rng.standard_normal(shape)
+    got = b200_fft_run(b200, psi0, v, step, mass, time, 2, prec=prec)
+    want = psi0.copy()
+    for _ in range(2):
+        want = restate.fft_step(want, step, mass, time, vc=v)
+    assert rel(got, want) < tol
+
+
 def test_split_step_no_potential(b200, restate):
     shape, step, mass = (16, 8, 32), 0.3, 1.0
     psi0 = smooth_state(shape, step)
