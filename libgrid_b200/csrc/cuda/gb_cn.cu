@@ -9,19 +9,22 @@
 // ends; the periodic case uses the Sherman-Morrison form of
 // grid_solve_tridiagonal_system_cyclic2 (src/linalg.c:206-230).
 //
-// Fast path (no absorbing region): every line of an axis sees the same matrix
-// (in a rotating frame: one matrix per perpendicular coordinate), so the elimination multipliers m_i, the reciprocal pivots
-// 1/b'_i and (periodic) the Sherman-Morrison vector z are computed once on
-// the host and each line needs only the right-hand side, one forward and one
-// backward sweep.  A CTA is one warp that owns up to 32 lines: the tile is
-// brought into shared memory with bulk asynchronous copies (one mbarrier,
-// bounded wait), the optional potential half-step is applied in place, each
-// lane sweeps its line, the second potential half-step is applied and the
-// tile is written back with bulk copies.  Contiguous (z) lines are padded by
-// one element in shared memory so the lane-per-line accesses hit distinct
-// banks; strided (x, y) tiles hold 32 adjacent columns per row.
+// Fast path (no absorbing region): every line of an axis sees the same matrix,
+// so the elimination multipliers m_i, the reciprocal pivots 1/b'_i and
+// (periodic) the Sherman-Morrison vector z are computed once, on the host, and
+// in a rotating frame, with one matrix per perpendicular coordinate, once per
+// matrix on the device; each line needs only the right-hand side, one forward
+// and one backward sweep.  A CTA of 16 warps owns up to 32 lines, each warp a
+// segment of every line (k_cn_fast): the tile is brought into shared memory with
+// bulk asynchronous copies (one mbarrier, bounded wait), the optional potential
+// half-step is applied in place, the lines are swept, the second potential
+// half-step is applied and the tile is written back with bulk copies.
+// Contiguous (z) lines are padded by one element in shared memory so the
+// lane-per-line accesses hit distinct banks; strided (x, y) tiles hold up to 32
+// adjacent columns per row.
 //
-// General path (absorbing boundary): one thread per line with per-element pivots in a global workspace laid out [i][line].
+// General path (absorbing boundary): one thread per line with per-element pivots
+// in a global workspace laid out [i][line].
 #include <complex>
 #include <math.h>
 #include <string.h>
@@ -191,7 +194,7 @@ __device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int 
 // at a time, lanes along the line.  Strided tiles (element (l, i) at
 // sm[i * pitch + l], pitch >= cols): one column per thread, `cols` columns
 // side by side, threads of equal column spaced along the rows.
-template <bool CONTIG>
+template <bool CONTIG, bool ZROWS = false>
 __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, int nl, long line0, long o, long col0,
                                             const CnAxis &a, const gb_potential &pt) {
   const int n = (int) a.n, nthr = (int) blockDim.x;
@@ -202,8 +205,14 @@ __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, in
       // lines along z; without a z axis (nz = 1) they run along y, or along x
       // when ny = 1 too, and their elements lie a potential row apart.  One
       // call for both: a second inlined copy cost 2% of a 192^3 step
-      long ix = a.axis == 1 ? lid : 0, iy = 0, vstep = vrow;
-      if (a.axis == 2) ix = lid / a.ny, iy = lid - ix * a.ny, vstep = 1;
+      long ix = 0, iy = 0, vstep = 1;
+      if (ZROWS || a.axis == 2) {
+        ix = lid / a.ny;
+        iy = lid - ix * a.ny;
+      } else {
+        if (a.axis == 1) ix = lid;
+        vstep = vrow;
+      }
       cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, (ix * a.ny + iy) * vrow, vstep, ix, iy, 0,
                    a, pt);
     }
@@ -278,12 +287,19 @@ template <int SMAX, class F> __device__ __forceinline__ void seg_loop_rev(int cn
   }
 }
 
-// CLS: lines of different matrices (a rotating frame, whose x and y sweeps
-// carry a coefficient proportional to the perpendicular coordinate).  The
-// tables then hold one set per coordinate, a lane reads those of its line,
-// and no rows are taken from registers.
-template <bool CONTIG, int SMAX, bool CLS>
+// Forms of the kernel.  kWhole: whole tiles (strided) or lines along z
+// (contiguous), never overlapped; tile width and potential stride are then the
+// launch's, and there is no wait, which 64 registers a thread just hold: 192^3
+// 331.6 us a step against 335.0 by kAny, 256 x 256 x 64 261.6 / 266.8.  kAny:
+// partial tiles, any contiguous axis, overlapped launches.  kRotating: kAny with
+// lines of different matrices (a rotating frame, whose x and y sweeps carry a
+// coefficient proportional to the perpendicular coordinate).  The tables then
+// hold one set per coordinate, a lane reads those of its line, and no rows are
+// taken from registers.
+enum { kWhole, kAny, kRotating };
+template <bool CONTIG, int SMAX, int FORM>
 __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ psi, CnAxis a) {
+  constexpr bool CLS = FORM == kRotating, ZROWS = FORM == kWhole;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) uint64_t bar;
   // segment end values, replaced in place by the segments' carries
@@ -303,8 +319,11 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
   } else {
     o = blockIdx.y;
     col0 = (long) blockIdx.x * lpc;
-    const long rem = a.inner - col0;
-    nl = (int) (rem < lpc ? rem : lpc);
+    nl = lpc;
+    if constexpr (FORM != kWhole) {
+      const long rem = a.inner - col0;
+      nl = (int) (rem < lpc ? rem : lpc);
+    }
   }
   const double2 zero = make_double2(0.0, 0.0);
 
@@ -315,7 +334,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
     mbar_arrive_expect_tx(&bar, (unsigned) (nl * n * 16));
   }
   __syncthreads();
-  grid_wait(psi);
+  if constexpr (FORM != kWhole) grid_wait(psi);
   if constexpr (CONTIG) {
     for (int l = tid; l < nl; l += 32 * kSeg) bulk_g2s(sm + (long) l * row, psi + (line0 + l) * n, (unsigned) (n * 16), &bar);
   } else {
@@ -330,7 +349,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
 
   // ---- optional first potential half-step (all threads, element-parallel)
   if (a.pre.kind != GB_POT_NONE || a.pre.g != 0.0)
-    cn_tile_pot<CONTIG>(sm, (int) row, lpc, nl, line0, o, col0, a, a.pre);
+    cn_tile_pot<CONTIG, ZROWS>(sm, (int) row, lpc, nl, line0, o, col0, a, a.pre);
   __syncthreads();
 
   const double2 *tab = a.tab;
@@ -445,7 +464,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2) k_cn_fast(double2 *__restrict__ 
   // ---- optional second potential half-step (element-parallel)
   if (a.post.kind != GB_POT_NONE || a.post.g != 0.0) {
     __syncthreads();
-    cn_tile_pot<CONTIG>(sm, (int) row, lpc, nl, line0, o, col0, a, a.post);
+    cn_tile_pot<CONTIG, ZROWS>(sm, (int) row, lpc, nl, line0, o, col0, a, a.post);
   }
 
   // ---- tile store
@@ -1164,30 +1183,46 @@ static int launch_cn_warp(void *psi, CnAxis &a, bool contig, int axis, cudaStrea
 
 }  // namespace
 
+// The fast kernel unrolled for the segment length of lines of n points.
+using FastKernel = void (*)(double2 *, CnAxis);
+template <bool CONTIG, int FORM> static FastKernel fast_kernel(long n) {
+  const long S = (n + kSeg - 1) / kSeg;
+  if (S <= 4) return k_cn_fast<CONTIG, 4, FORM>;
+  if (S <= 8) return k_cn_fast<CONTIG, 8, FORM>;
+  if (S <= 12) return k_cn_fast<CONTIG, 12, FORM>;
+  if (S <= 16) return k_cn_fast<CONTIG, 16, FORM>;
+  return k_cn_fast<CONTIG, 0, FORM>;
+}
+
+// One sweep.  Small sweeps overlap the end of the one before; with more waves
+// of CTAs (two on each SM) those that wait only take slots.  One step, launch by
+// launch / overlapped up to one and a half waves / up to two, us: 64^3 41.8 /
+// 35.4 / 35.4; 96^3 55.8 / 50.7 / 50.7; 112^3 104.6 / 104.3 / 102.8; 120^3
+// 105.4 / 105.1 / 107.5; 128^3 110.9 / 110.8 / 111.4; 136^3 131.4 / 131.4 /
+// 133.2.  In a rotating frame, whose sweeps wait longer for their tables: 96^3
+// 61.7 / 55.0 / 54.9; 120^3 119.4 / 119.1 / 114.8; 128^3 125.5 / 125.0 / 119.7;
+// 136^3 151.8 / 151.8 / 149.7, up to three waves 147.7; 144^3 196.9 / 198.7 /
+// 198.3, 196.1.  A sweep right after the kernel that built its tables (built)
+// does not overlap it: the tables are read as constants.
+template <bool CONTIG>
+static int cn_launch(dim3 grid, size_t smem, cudaStream_t st, void *psi, const CnAxis &a, bool cls, bool built) {
+  const long wave = 2 * gb__num_sms();
+  const bool overlap = !built && (long) grid.x * grid.y <= (cls ? 2 * wave : wave + wave / 2);
+  const bool whole = CONTIG ? a.axis == 2 : a.inner % a.lpc == 0;
+  const FastKernel kern = cls                 ? fast_kernel<CONTIG, kRotating>(a.n)
+                          : whole && !overlap ? fast_kernel<CONTIG, kWhole>(a.n)
+                                              : fast_kernel<CONTIG, kAny>(a.n);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+  const int slot = gb__pass_begin(15 + a.axis);
+  launch_stream(overlap, kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
+  gb__pass_end(slot);
+  GB_CHECK_LAUNCH("cn fast");
+  return 0;
+}
+
 // Warp-cooperative line solver on (1) or off (0, the default: the
 // segment-per-warp kernel, measured faster on B200 at 192^3: 0.447 against
 // 0.487 ms per step); -1 only queries.
-// The fast kernel unrolled for the segment length of lines of n points.
-using FastKernel = void (*)(double2 *, CnAxis);
-template <bool CONTIG, bool CLS> static FastKernel fast_kernel(long n) {
-  const long S = (n + kSeg - 1) / kSeg;
-  if (S <= 4) return k_cn_fast<CONTIG, 4, CLS>;
-  if (S <= 8) return k_cn_fast<CONTIG, 8, CLS>;
-  if (S <= 12) return k_cn_fast<CONTIG, 12, CLS>;
-  if (S <= 16) return k_cn_fast<CONTIG, 16, CLS>;
-  return k_cn_fast<CONTIG, 0, CLS>;
-}
-
-// Sweeps of up to two waves (two CTAs on each of 148 SMs) overlap the end of
-// the one before: 100 x 100 x 50 in a rotating frame 70.8 -> 66.6 us a step,
-// 125 x 99 x 75 82.9 -> 81.9 us.  With more waves the waiting CTAs only take
-// slots: 192^3 (four waves) 341.1 -> 343.2 us.  A sweep right after the kernel
-// that built its tables does not overlap it: the tables are read as constants.
-static void cn_launch(FastKernel kern, dim3 grid, size_t smem, cudaStream_t st, void *psi, const CnAxis &a, bool built) {
-  const bool overlap = !built && (long) grid.x * grid.y <= 2 * 296;
-  launch_stream(overlap, kern, grid, 32 * kSeg, smem, st, (double2 *) psi, a);
-}
-
 static int g_cn_warp_on = 0;
 extern "C" int gb_cn_warp_solver(int on) {
   const int old = g_cn_warp_on;
@@ -1301,8 +1336,8 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&smpm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         cudaFuncAttributes fa0, fa1;
-        cudaFuncGetAttributes(&fa0, k_cn_fast<true, 0, false>);
-        cudaFuncGetAttributes(&fa1, k_cn_fast<false, 0, false>);
+        cudaFuncGetAttributes(&fa0, k_cn_fast<true, 0, kAny>);
+        cudaFuncGetAttributes(&fa1, k_cn_fast<false, 0, kAny>);
         const size_t st_max = fa0.sharedSizeBytes > fa1.sharedSizeBytes ? fa0.sharedSizeBytes : fa1.sharedSizeBytes;
         const long b = (long) smpm / 2 - 1024 - (long) st_max;
         budget = b > 16 * 1024 ? (size_t) b : 16 * 1024;
@@ -1314,14 +1349,8 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         if (lpc < 1) return gb__set_error(1011, "cn: line too long for a shared-memory tile");
         a.lpc = (int) lpc;
         const size_t sm = (size_t) lpc * row * 16;
-        const FastKernel kern = cls ? fast_kernel<true, true>(a.n) : fast_kernel<true, false>(a.n);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         const long nb = (a.outer + lpc - 1) / lpc;
-        {
-          const int slot = gb__pass_begin(15 + axis);
-          cn_launch(kern, dim3((unsigned) nb), sm, st, psi, a, built);
-          gb__pass_end(slot);
-        }
+        GB_TRYC(cn_launch<true>(dim3((unsigned) nb), sm, st, psi, a, cls, built));
       } else {
         long cap = (long) (budget / (a.n * 16));
         if (cap > 32) cap = 32;
@@ -1332,17 +1361,10 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
         const long lpc = pow2_at_most(cap);
         a.lpc = (int) lpc;
         const size_t sm = (size_t) lpc * a.n * 16;
-        const FastKernel kern = cls ? fast_kernel<false, true>(a.n) : fast_kernel<false, false>(a.n);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);
         if (a.outer > 65535) return gb__set_error(1012, "cn: outer extent above 65535");
         dim3 grid((unsigned) ((a.inner + lpc - 1) / lpc), (unsigned) a.outer);
-        {
-          const int slot = gb__pass_begin(15 + axis);
-          cn_launch(kern, grid, sm, st, psi, a, built);
-          gb__pass_end(slot);
-        }
+        GB_TRYC(cn_launch<false>(grid, sm, st, psi, a, cls, built));
       }
-      GB_CHECK_LAUNCH("cn fast");
     } else {
       if (a.pre.kind != GB_POT_NONE || a.pre.g != 0.0) GB_TRYC(gb_potential_multiply(psi, g, &a.pre));
       double2 *work = (double2 *) gb__scratch(GB_SCR_WORK, sizeof(double2) * (size_t) nxyz * 4);

@@ -24,6 +24,7 @@ enum {
   GB_SCR_COUNT = 14
 };
 
+int gb__num_sms(void);  // of the current device
 void *gb__scratch(int slot, size_t bytes);
 // Tables kept from call to call under a key of the call's parameters.  A kept
 // table counts while gb__table_gen() is what it was when the table was built

@@ -313,6 +313,17 @@ extern "C" float gb_event_elapsed_ms(int a, int b) {
   return ms;
 }
 
+int gb__num_sms(void) {
+  static int dev_known = -1, n = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev != dev_known) {
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    dev_known = dev;
+  }
+  return n;
+}
+
 void *gb__scratch(int slot, size_t bytes) {
   if (slot < 0 || slot >= GB_SCR_COUNT) return nullptr;
   Scratch &s = g_scratch[slot];

@@ -672,13 +672,6 @@ int pow2_at_least(int v) {
   return p;
 }
 
-int num_sms() {
-  int nsm = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return nsm;
-}
-
 // Block shape: the candidate with the least estimated time.  A CTA alone
 // spends about 46 cycles per warp item of staging, 34 per MMA, 360 per M-tile
 // of the epilogue and 4400 besides; CTAs that share an SM overlap each other's
@@ -932,7 +925,7 @@ extern "C" int gb_unet_tensor_cores(int on) {
 int gb__unet_conv_tc(const float *x, const uint16_t *w, const float *b, float *y, int cin, int cout, int nb, int d,
                      int h, int wd, int relu, int mode) {
   if (!g_tc_on) return -1;
-  const int nsm = num_sms();
+  const int nsm = gb__num_sms();
   TcPlan pl;
   if (!tc_plan(mode == 0 ? cin : cout, mode == 0 ? cout : cin, nb, d, h, wd, nsm, pl)) return -1;
   return run_conv_tc(pl, nsm, x, w, b, y, cin, cout, nb, d, h, wd, relu, mode);

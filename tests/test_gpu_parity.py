@@ -270,6 +270,23 @@ def test_cn_step_short_axes(b200, restate, bc, shape, gp):
         assert rel(got, want) < TOL_PSI
 
 
+@pytest.mark.parametrize("bc", [DIR, NEU, PER])
+@pytest.mark.parametrize("shape", [(512, 4, 32), (512, 30, 4), (6, 500, 32), (6, 500, 31), (1000, 16, 1)])
+def test_cn_many_tiles(b200, restate, bc, shape):
+    """Sweeps of more CTAs than overlap, along each axis, of whole tiles and
+    with a partial last one, with real and complex potentials."""
+    step, mass, g = 0.3, 4.0 / workloads.GRID_AUTOAMU, 0.001
+    psi0, v = workloads.cn_wells(shape, step, g, seed=13)
+    got = b200_cn_run(b200, psi0, None, step, mass, 0.5, bc, 2, gp=(v, g))
+    want = psi0.copy()
+    for _ in range(2):
+        want = restate.cn_step(want, step, mass, 0.5, bc, vr=workloads.padded(v), g=g)
+    assert rel(got, want) < TOL_PSI
+    vc = v + 1e-4j * np.cos(np.arange(v.size)).reshape(shape)
+    got = b200_cn_run(b200, psi0, vc, step, mass, 0.5, bc, 1)
+    assert rel(got, restate.cn_step(psi0.copy(), step, mass, 0.5, bc, vc=vc)) < TOL_PSI
+
+
 @pytest.mark.parametrize("bc", [DIR, PER])
 def test_cn_rotation_and_absorber(b200, restate, bc):
     """General line-solver path: rotating frame and absorbing ramp."""
