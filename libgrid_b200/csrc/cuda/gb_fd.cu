@@ -7,11 +7,13 @@
 // lands outside the grid again (the reference recurses without end there);
 // this implementation uses the single plane instead.
 //
-// Stencils read their neighbours directly, one output element per thread and
-// load batch (k_fd below).  Laplacian sums keep the reference's left-to-right
+// Stencils read their neighbours directly, two or four output elements per thread
+// with their loads issued together (k_fd below).  Laplacian sums keep the reference's left-to-right
 // order
 //   (-6 c + z+ + z- + y+ + y- + x+ + x-) / h^2     (src/cgrid_diff.c:330-335).
 #include <string.h>
+
+#include <algorithm>
 
 #include "gb_common.cuh"
 #include "gb_internal_cuda.h"
@@ -101,8 +103,8 @@ __device__ __forceinline__ typename Elem<T, REAL>::V neighbour(const typename El
   return src[idx - c * s + m * s];
 }
 
-// Element e of the grid's nx * ny * nz points: its storage index and its
-// neighbours along the axes that MODE takes (0, 1, 2: x, y, z; 3: all, in the
+// Element e of the grid's nx * ny * nz points: its storage index (both below
+// 2^31) and its neighbours along the axes that MODE takes (0, 1, 2: x, y, z; 3: all, in the
 // order z+, z-, y+, y-, x+, x-).
 template <typename T, bool REAL, int MODE, typename I>
 __device__ __forceinline__ I fd_load(typename Elem<T, REAL>::V (&nb)[MODE == 3 ? 6 : 2],
@@ -129,11 +131,12 @@ __host__ __device__ constexpr int fd_unroll(int mode) { return mode == 3 ? 2 : 4
 
 // MODE 0, 1, 2: second difference (lap) or central difference along x, y, z;
 // MODE 3: the seven-point Laplacian.
-template <typename T, bool REAL, int MODE, typename I>
+template <typename T, bool REAL, int MODE>
 __global__ void __launch_bounds__(kFdThreads) k_fd(bool lap, typename Elem<T, REAL>::V *__restrict__ dst,
                                                    const typename Elem<T, REAL>::V *__restrict__ src, FdArgs a) {
   using E = Elem<T, REAL>;
   using V = typename E::V;
+  using I = unsigned;
   constexpr int U = fd_unroll(MODE), NB = MODE == 3 ? 6 : 2;
   const I total = (I) a.nx * (I) a.ny * (I) a.nz;
   const I e0 = (I) blockIdx.x * (I) (kFdThreads * U) + (I) threadIdx.x;
@@ -160,6 +163,96 @@ __global__ void __launch_bounds__(kFdThreads) k_fd(bool lap, typename Elem<T, RE
         r = E::sub(nb[u][0], nb[u][1]);
       }
       dst[idx[u]] = E::scale(r, (T) a.coef);
+    }
+  }
+}
+
+// The same over bands of rows: a CTA takes consecutive elements of the band j0 ..
+// j0 + rows - 1 of plane i, the CTAs go along x within a band.  Offsets within
+// the band and coordinates are of type N; the plane's x neighbours and the row and
+// column shifts are pointers of the whole CTA.
+struct FdBands {
+  unsigned rows, cpb;  // rows of a band, CTAs of a band of one plane
+};
+
+// The neighbour below (DIR < 0) or above along y or z at p[off]; outside the axis
+// by the boundary rule, as an offset of c, n, s (coordinate, points, stride).
+template <int DIR, typename T, bool REAL, typename N>
+__device__ __forceinline__ typename Elem<T, REAL>::V band_neighbour(const typename Elem<T, REAL>::V *__restrict__ p,
+                                                                    N off, N c, N n, long s, const FdArgs &a) {
+  if (DIR > 0 ? c + 1 < n : c > 0) return p[off];
+  if (a.bc == GB_BC_DIRICHLET) return Elem<T, REAL>::outside(a.out_re, a.out_im);
+  N m;  // the coordinate that stands for the outside one
+  if (a.bc == GB_BC_PERIODIC) m = DIR > 0 ? 0 : n - 1;
+  else m = n == 1 ? 0 : DIR > 0 ? n - 2 : 1;
+  return (p + ((long) m - (long) c - DIR) * s)[off];
+}
+
+template <typename T, bool REAL, int MODE, typename N>
+__global__ void __launch_bounds__(kFdThreads) k_fd_bands(bool lap, typename Elem<T, REAL>::V *__restrict__ dst,
+                                                         const typename Elem<T, REAL>::V *__restrict__ src, FdArgs a,
+                                                         FdBands b) {
+  using E = Elem<T, REAL>;
+  using V = typename E::V;
+  constexpr int U = fd_unroll(MODE), NB = MODE == 3 ? 6 : 2, Y = MODE == 3 ? 2 : 0, X = MODE == 3 ? 4 : 0;
+  const unsigned q = blockIdx.x / b.cpb, band = q / (unsigned) a.nx, i = q - band * (unsigned) a.nx;
+  const N nz = (N) a.nz, ny = (N) a.ny, row = (N) a.row, j0 = (N) band * b.rows;
+  const N total = min((N) b.rows, ny - j0) * nz;
+  const N e0 = (N) (blockIdx.x - q * b.cpb) * (N) (kFdThreads * U) + threadIdx.x;
+  const long plane = a.ny * a.row, base = (long) i * plane + (long) j0 * a.row;
+  const V *s = src + base;
+  V *d = dst + base;
+  // planes i + 1 and i - 1, or the ones that stand for them
+  const V *xp = s + plane, *xm = s - plane;
+  bool xp_out = false, xm_out = false;
+  if (MODE == 0 || MODE == 3) {
+    const long nx = a.nx;
+    if (i + 1 == nx) {
+      xp_out = a.bc == GB_BC_DIRICHLET;
+      xp = s + ((a.bc == GB_BC_PERIODIC || nx == 1 ? 0 : nx - 2) - (long) i) * plane;
+    }
+    if (i == 0) {
+      xm_out = a.bc == GB_BC_DIRICHLET;
+      xm = s + (a.bc == GB_BC_PERIODIC ? nx - 1 : nx == 1 ? 0 : 1) * plane;
+    }
+  }
+  const bool centre = MODE == 3 || lap;
+  V c[U], nb[U][NB];
+  N off[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const N e = e0 + (N) (u * kFdThreads);
+    if (e < total) {
+      const N r = e / nz, k = e - r * nz;
+      const N o = r * row + k;
+      off[u] = o;
+      if constexpr (MODE >= 2) {
+        nb[u][0] = band_neighbour<1, T, REAL, N>(s + 1, o, k, nz, 1, a);
+        nb[u][1] = band_neighbour<-1, T, REAL, N>(s - 1, o, k, nz, 1, a);
+      }
+      if constexpr (MODE == 1 || MODE == 3) {
+        nb[u][Y] = band_neighbour<1, T, REAL, N>(s + a.row, o, j0 + r, ny, a.row, a);
+        nb[u][Y + 1] = band_neighbour<-1, T, REAL, N>(s - a.row, o, j0 + r, ny, a.row, a);
+      }
+      if constexpr (MODE == 0 || MODE == 3) {
+        nb[u][X] = xp_out ? E::outside(a.out_re, a.out_im) : xp[o];
+        nb[u][X + 1] = xm_out ? E::outside(a.out_re, a.out_im) : xm[o];
+      }
+      if (centre) c[u] = s[o];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    if (e0 + (N) (u * kFdThreads) < total) {
+      V r;
+      if (centre) {
+        r = E::scale(c[u], (T) (MODE == 3 ? -6.0 : -2.0));
+#pragma unroll
+        for (int w = 0; w < NB; w++) r = E::add(r, nb[u][w]);
+      } else {
+        r = E::sub(nb[u][0], nb[u][1]);
+      }
+      d[off[u]] = E::scale(r, (T) a.coef);
     }
   }
 }
@@ -373,15 +466,42 @@ int fd_grid(const gb_geom *g, dim3 *grid) {
   return 0;
 }
 
-// 32-bit indices up to 2^31 stored elements less the overhang of a launch: the
-// two divisions of a point cost several times as much in 64 bits.
+// Flat order up to 2^31 stored elements less the overhang of a launch: the two
+// divisions of a point cost several times as much in 64 bits.  Beyond, and where
+// the planes that an x neighbour takes are too large for L2 to hold three of, in
+// bands: at 1300^3 (2.2e9 points) flat with 64-bit indices / bands, ms: Laplacian
+// 31.0 / 15.3 complex, 17.4 / 11.2 real FP32; x gradient 16.2 / 10.7, 10.6 / 5.1;
+// z gradient 11.7 / 10.3, 7.2 / 5.3 (halo tiles 17.7 and 11.6 throughout).  Complex
+// FP64 Laplacian, flat / bands, us: 96 x 1024 x 1024 (planes of 17 MB) 669 / 705;
+// 80 x 1150 x 1150 (21 MB) 781 / 773; 64 x 1300 x 1300 (27 MB) 947 / 764; 32 x
+// 2048 x 2048 (67 MB) 1181 / 947; x gradient there 914 / 666, y 625 / 652.
+// Elements of 8 bytes: Laplacian 690 / 732 at 32 x 2048 x 2048.  Bands of 8 MB in
+// place of 2: 825 at 64 x 1300 x 1300; where three planes fit, whole planes (1300^3
+// real FP32 Laplacian 11.2 ms against 12.5 in bands of 2 MB).
+constexpr long kFdBandPlane = 20L << 20, kFdBandBytes = 2L << 20;
+
 template <typename T, bool REAL, int MODE>
 int fd_launch(bool lap, void *dst, const void *src, const FdArgs &a) {
   using V = typename Elem<T, REAL>::V;
-  const long per = (long) kFdThreads * fd_unroll(MODE), nb = (a.nx * a.ny * a.nz + per - 1) / per;
-  const bool w32 = a.nx * a.ny * a.row < (1L << 31) - (1L << 20);
-  auto kern = w32 ? k_fd<T, REAL, MODE, unsigned> : k_fd<T, REAL, MODE, unsigned long>;
-  kern<<<(unsigned) nb, kFdThreads, 0, gb__stream()>>>(lap, (V *) dst, (const V *) src, a);
+  constexpr long CH = (long) kFdThreads * fd_unroll(MODE), kMost = (1L << 31) - (1L << 20);
+  const long plane = a.ny * a.row, row_bytes = a.row * (long) sizeof(V);
+  V *d = (V *) dst;
+  const V *s = (const V *) src;
+  cudaStream_t st = gb__stream();
+  const bool along_x = (MODE == 0 || MODE == 3) && sizeof(V) == 16;
+  if (a.nx * plane < kMost && !(along_x && plane * (long) sizeof(V) > kFdBandPlane)) {
+    const long nb = (a.nx * a.ny * a.nz + CH - 1) / CH;
+    k_fd<T, REAL, MODE><<<(unsigned) nb, kFdThreads, 0, st>>>(lap, d, s, a);
+  } else {
+    FdBands b;
+    const long want = plane * (long) sizeof(V) <= kFdBandPlane ? a.ny : std::max(8L, kFdBandBytes / row_bytes);
+    const long rows = std::max(1L, std::min(std::min(a.ny, want), kMost / a.row));
+    b.rows = (unsigned) rows;
+    b.cpb = (unsigned) ((rows * a.nz + CH - 1) / CH);
+    const unsigned nb = (unsigned) ((a.ny + rows - 1) / rows * a.nx * b.cpb);
+    if (a.row < kMost) k_fd_bands<T, REAL, MODE, unsigned><<<nb, kFdThreads, 0, st>>>(lap, d, s, a, b);
+    else k_fd_bands<T, REAL, MODE, unsigned long><<<nb, kFdThreads, 0, st>>>(lap, d, s, a, b);
+  }
   GB_CHECK_LAUNCH("fd stencil");
   return 0;
 }

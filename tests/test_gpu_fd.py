@@ -1,6 +1,6 @@
 """Finite-difference stencils and the FD kinetic energy against numpy, over
-the boundary rules, odd sizes, axes of one and two points, and grids below and
-above one chunk of a launch."""
+the boundary rules, odd sizes, axes of one and two points, grids below and above
+one chunk of a launch, planes that go in bands, and more points than 32 bits."""
 import ctypes as C
 
 import numpy as np
@@ -42,8 +42,9 @@ def _close(got, want, scale):
     assert np.abs(got - want).max() <= 16 * 2.3e-16 * scale
 
 
+# the last two: planes above 20 MB, taken in bands of rows (the last one partial)
 @pytest.mark.parametrize("bc", ["dirichlet", "neumann", "periodic"])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + [(3, 1153, 1151), (1, 9, 150001)])
 def test_stencils(b200, shape, bc):
     rng, step = np.random.default_rng(sum(shape)), 0.3
     a = rng.uniform(-1, 1, shape) + 1j * rng.uniform(-1, 1, shape)
@@ -74,3 +75,54 @@ def test_kinetic_energy(b200, shape, bc, boundary):
     kinetic.restype = C.c_double
     assert abs(kinetic(w.ptr) - want) <= 1e-12 * abs(want)
     b200.free(w)
+
+
+class _Geom(C.Structure):
+    _fields_ = [("nx", C.c_long), ("ny", C.c_long), ("nz", C.c_long), ("step", C.c_double), ("prec", C.c_int)]
+
+
+@pytest.mark.parametrize("bc", [1, 2])  # Neumann, periodic
+@pytest.mark.parametrize("shape", [(131072, 128, 127), (2, 32771, 32769)])
+def test_more_points_than_32_bits(b200, shape, bc):
+    """Real FP32 grids of 2.1e9 stored elements, with small planes and with
+    planes of 4.3 GB, checked on planes and rows at the edges and inside."""
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = shape
+    lib, row = b200.lib, 2 * (nz // 2 + 1)
+    assert nx * ny * row >= 2**31
+    lib.cuda_enable(b"\x01", 0, None)
+    lib.gb_fd.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.POINTER(_Geom), C.c_int] + 3 * [C.c_double] + [C.c_int, C.c_long]
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    a = torch.rand((nx, ny, row), generator=gen, device="cuda")
+    out = torch.empty_like(a)
+    g = _Geom(nx, ny, nz, 0.3, 1)
+    ii = sorted({0, 1, nx // 2, nx - 1})
+    jj = sorted({0, 1, ny // 2, ny - 1})
+
+    def shift(c, n):  # coordinate that stands for c
+        if bc == 2:
+            return c % n
+        return -c if c < 0 else (2 * n - 2 - c if c > n - 1 else c)
+
+    kp = torch.tensor([shift(k + 1, nz) for k in range(nz)], device="cuda")
+    km = torch.tensor([shift(k - 1, nz) for k in range(nz)], device="cuda")
+    for op, axes, lap in ((1, (2, 1, 0), 1), (2, (0,), 1), (3, (1,), 1), (4, (2,), 1), (5, (0,), 0), (6, (1,), 0), (7, (2,), 0)):
+        torch.cuda.synchronize()
+        assert lib.gb_fd(op, out.data_ptr(), a.data_ptr(), C.byref(g), bc, 0.0, 0.0, 0.5, 1, row) == 0
+        assert lib.gb_synchronize() == 0
+        for i in ii:
+            for j in jj:
+                c = a[i, j, :nz].double()
+                want = -2.0 * len(axes) * c if lap else torch.zeros_like(c)
+                for d in axes:
+                    if d == 2:
+                        p, m = c[kp], c[km]
+                    elif d == 1:
+                        p, m = a[i, shift(j + 1, ny), :nz].double(), a[i, shift(j - 1, ny), :nz].double()
+                    else:
+                        p, m = a[shift(i + 1, nx), j, :nz].double(), a[shift(i - 1, nx), j, :nz].double()
+                    want += p + m if lap else p - m
+                # up to eight terms of at most six times the largest value
+                assert (out[i, j, :nz].double() - 0.5 * want).abs().max() <= 16 * 6e-8 * 6 * 0.5
+    del a, out
+    torch.cuda.empty_cache()
