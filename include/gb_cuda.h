@@ -92,6 +92,10 @@ int gb_graph_begin(void);
 int gb_graph_end(void **graph);
 int gb_graph_launch(void *graph);
 int gb_graph_free(void *graph);
+/* Largest scratch buffer or table that the library allocates from now on
+ * (0, the default: no limit); returns the setting before.  A call that cannot do
+ * with less fails as when device memory runs out. */
+size_t gb_scratch_limit(size_t bytes);
 void *gb_device_alloc(size_t bytes);
 void gb_device_free(void *p);
 void *gb_host_alloc(size_t bytes); /* page-locked when possible */

@@ -1093,24 +1093,28 @@ struct CnClassKey {
 };
 static CnClassKey g_cls_key[2];
 
-static double2 *class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off,
-                             bool *built) {
+// *tab: the tables, null when there is no memory for them; *built: whether this
+// call built them.
+static int class_tables(int axis, long n, long ncls, int bc, cd cp, cd c2, cd c3, double step, double off,
+                        const double2 **tab, bool *built) {
   CnClassKey &k = g_cls_key[axis];
   *built = false;
+  *tab = k.tab;
   if (k.gen == gb__table_gen() && k.n == n && k.ncls == ncls && k.bc == bc && k.cp == cp && k.c2 == c2 && k.c3 == c3 &&
       k.step == step && k.off == off)
-    return k.tab;
+    return 0;
   cudaStream_t st;
   k.gen = 0;
-  double2 *tab = (double2 *) gb__table_alloc(axis == 0 ? GB_SCR_CNROT0 : GB_SCR_CNROT1,
-                                             sizeof(double2) * (size_t) (cls_pitch(n) * ncls), &st);
-  if (!tab) return nullptr;
+  double2 *t = (double2 *) gb__table_alloc(axis == 0 ? GB_SCR_CNROT0 : GB_SCR_CNROT1,
+                                           sizeof(double2) * (size_t) (cls_pitch(n) * ncls), &st, false);
+  *tab = t;
+  if (!t) return 0;
   auto v2 = [](cd z) { return make_double2(z.real(), z.imag()); };
-  k_cn_class_tables<<<(unsigned) ((ncls + 31) / 32), 32, 0, st>>>(tab, n, ncls, bc, v2(cp), v2(c2), v2(c3), step, off);
-  if (gb__table_built(st, "cn class tables")) return nullptr;
+  k_cn_class_tables<<<(unsigned) ((ncls + 31) / 32), 32, 0, st>>>(t, n, ncls, bc, v2(cp), v2(c2), v2(c3), step, off);
+  GB_TRYC(gb__table_built(st, "cn class tables"));
   *built = true;
-  k = CnClassKey{gb__table_gen(), tab, n, ncls, bc, cp, c2, c3, step, off};
-  return tab;
+  k = CnClassKey{gb__table_gen(), t, n, ncls, bc, cp, c2, c3, step, off};
+  return 0;
 }
 
 // Persistent launch of the warp-cooperative kernel: one resident wave of
@@ -1307,26 +1311,27 @@ extern "C" int gb_cn_step(void *psi, const gb_geom *g, const gb_cn_params *p, co
     // in a rotating frame the matrix of an x (y) line depends on its y (x)
     const bool cls = c3 != cd(0.0);
     // a rotating frame goes on to the general path, which keeps no tables,
-    // where the tiles or the tables (up to 1 GB) of the fast one end and in a
-    // capture whose graph cannot hold tables; without rotation those are errors
+    // where the tiles or the tables (up to 1 GB) of the fast one end, where there
+    // is no memory for them, and in a capture whose graph cannot hold them;
+    // without rotation those are errors
+    const cd cp = c / tstep;
     const long ncls = axis == 0 ? g->ny : g->nx;
-    const bool fast = !p->absorb && (p->omega == 0.0 || (a.n <= kFastMaxN && (contig || a.outer <= 65535) &&
-                                                         (!cls || cls_pitch(a.n) * ncls <= (1L << 26)) &&
-                                                         !gb__foreign_capture()));
+    bool fast = !p->absorb && (p->omega == 0.0 || (a.n <= kFastMaxN && (contig || a.outer <= 65535) &&
+                                                   (!cls || cls_pitch(a.n) * ncls <= (1L << 26)) &&
+                                                   !gb__foreign_capture()));
+    bool built = false;
+    if (fast && cls) {
+      GB_TRYC(class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step, a.coord_off, &a.tab, &built));
+      fast = a.tab != nullptr;
+    }
     if (fast && !cls && a.n <= 32 * kLaneSegMax && g_cn_warp_on) {
-      const cd cp = c / tstep;
       double2 *tab = fast_tables(s, a.n, p->boundary, cp, c2, 32, &a);
       if (!tab) return gb_last_error();
       a.tab = tab;
       a.cp = make_double2(cp.real(), cp.imag());
       GB_TRYC(launch_cn_warp(psi, a, contig, axis, st));
     } else if (fast) {
-      const cd cp = c / tstep;
-      bool built = false;
-      double2 *tab = cls ? class_tables(axis, a.n, ncls, p->boundary, cp, c2, c3, g->step, a.coord_off, &built)
-                         : fast_tables(s, a.n, p->boundary, cp, c2, kSeg, &a);
-      if (!tab) return gb_last_error();
-      a.tab = tab;
+      if (!cls && !(a.tab = fast_tables(s, a.n, p->boundary, cp, c2, kSeg, &a))) return gb_last_error();
       a.cp = make_double2(cp.real(), cp.imag());
       // tile budget: two CTAs per SM, each with its tile, its static
       // shared memory and the per-CTA reservation

@@ -25,7 +25,8 @@ enum {
 };
 
 int gb__num_sms(void);  // of the current device
-void *gb__scratch(int slot, size_t bytes);
+// Without `must` a failed allocation sets no error.
+void *gb__scratch(int slot, size_t bytes, bool must = true);
 // Tables kept from call to call under a key of the call's parameters.  A kept
 // table counts while gb__table_gen() is what it was when the table was built
 // (it changes at gb_shutdown and where gb_graph_begin's capture starts and
@@ -33,7 +34,7 @@ void *gb__scratch(int slot, size_t bytes);
 // in a capture, memory of the graph, and the stream its building kernel goes
 // to; gb__table_built follows that launch.
 int gb__table_gen(void);
-void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st);
+void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st, bool must = true);
 int gb__table_built(cudaStream_t st, const char *where);
 // Whether the library stream is being captured by other means than
 // gb_graph_begin (the library then owns no memory of the graph).

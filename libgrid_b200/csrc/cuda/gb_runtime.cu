@@ -324,7 +324,25 @@ int gb__num_sms(void) {
   return n;
 }
 
-void *gb__scratch(int slot, size_t bytes) {
+static size_t g_alloc_limit = 0;  // gb_scratch_limit
+
+extern "C" size_t gb_scratch_limit(size_t bytes) {
+  const size_t old = g_alloc_limit;
+  g_alloc_limit = bytes;
+  return old;
+}
+
+// Device memory for scratch and tables; null when there is none (or more than
+// gb_scratch_limit is asked for).
+static void *scratch_alloc(size_t bytes) {
+  void *p = nullptr;
+  if (g_alloc_limit && bytes > g_alloc_limit) return nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
+void *gb__scratch(int slot, size_t bytes, bool must) {
   if (slot < 0 || slot >= GB_SCR_COUNT) return nullptr;
   Scratch &s = g_scratch[slot];
   if (s.bytes >= bytes && s.p) return s.p;
@@ -333,7 +351,7 @@ void *gb__scratch(int slot, size_t bytes) {
       // a live graph may hold this buffer's address: keep it until the last
       // graph is freed (a bounded list; beyond it the call fails instead)
       if (g_nretired >= 64) {
-        gb__set_error(2, "scratch: too many buffers replaced while CUDA graphs are alive");
+        if (must) gb__set_error(2, "scratch: too many buffers replaced while CUDA graphs are alive");
         return nullptr;
       }
       g_retired[g_nretired++] = s.p;
@@ -342,33 +360,25 @@ void *gb__scratch(int slot, size_t bytes) {
       cudaFree(s.p);
     }
   }
-  s.p = nullptr;
-  s.bytes = 0;
-  size_t want = bytes < 4096 ? 4096 : bytes;
-  if (cudaMalloc(&s.p, want) != cudaSuccess) {
-    cudaGetLastError();
-    gb__set_error(2, "scratch cudaMalloc");
-    s.p = nullptr;
-    return nullptr;
+  s.bytes = bytes < 4096 ? 4096 : bytes;
+  s.p = scratch_alloc(s.bytes);
+  if (!s.p) {
+    s.bytes = 0;
+    if (must) gb__set_error(2, "scratch cudaMalloc");
   }
-  s.bytes = want;
   return s.p;
 }
 
 int gb__table_gen(void) { return g_table_gen; }
 
 // Memory for a table about to be built, and the stream to build it on.
-void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st) {
+void *gb__table_alloc(int slot, size_t bytes, cudaStream_t *st, bool must) {
   *st = g_stream;
-  if (!g_capturing) return gb__scratch(slot, bytes);
+  if (!g_capturing) return gb__scratch(slot, bytes, must);
   *st = g_table_stream;
-  void *p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    gb__set_error(2, "graph: table cudaMalloc");
-    return nullptr;
-  }
-  g_capture_tables.push_back(p);
+  void *p = scratch_alloc(bytes);
+  if (p) g_capture_tables.push_back(p);
+  else if (must) gb__set_error(2, "graph: table cudaMalloc");
   return p;
 }
 

@@ -5,6 +5,8 @@ Tolerances (FP64 mode): psi relative L2 <= 1e-11, energies relative <= 1e-12
 (1e-10 absolute-relative for sums that cancel), norms relative <= 1e-12.
 FP32 mode is checked against the FP64 oracle with its stated error bound.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -340,6 +342,22 @@ def test_cn_rotation_changing(b200, restate, bc, shape):
     assert rel(w.grid.get(), want) < TOL_PSI
     b200.free(w)
     b200.free(pot)
+
+
+def test_cn_rotation_without_memory_for_tables(b200, restate):
+    """A rotating step whose tables (96 bytes a point of the plane) cannot be
+    allocated while the general path's workspace (64) can takes that path."""
+    lib, shape, step, mass, time = b200.lib, (901, 907, 1), 0.3, 1.0, 0.05
+    lib.gb_scratch_limit.restype, lib.gb_scratch_limit.argtypes = C.c_size_t, [C.c_size_t]
+    rng = np.random.default_rng(41)
+    psi0 = smooth_state(shape, step) + 0.01 * rand_c(rng, shape)
+    v = 0.02 * rng.standard_normal(shape).astype(complex)
+    old = lib.gb_scratch_limit(80 * shape[0] * shape[1])
+    try:
+        got = b200_cn_run(b200, psi0, v, step, mass, time, DIR, 1, omega=0.3)
+    finally:
+        lib.gb_scratch_limit(old)
+    assert rel(got, restate.cn_step(psi0.copy(), step, mass, time, DIR, omega=0.3, vc=v)) < TOL_PSI
 
 
 @pytest.mark.parametrize("bc", [DIR, NEU, PER])
