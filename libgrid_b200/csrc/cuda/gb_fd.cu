@@ -62,10 +62,9 @@ __device__ __forceinline__ bool map_index(long &i, long n, int bc) {
   return true;
 }
 
-template <typename T, bool REAL>
-__device__ __forceinline__ typename Elem<T, REAL>::V fetch(const typename Elem<T, REAL>::V *src, long i, long j, long k,
-                                                           const FdArgs &a) {
-  using E = Elem<T, REAL>;
+template <typename T>
+__device__ __forceinline__ C2<T> fetch(const C2<T> *src, long i, long j, long k, const FdArgs &a) {
+  using E = Elem<T, false>;
   if (i < 0 || i >= a.nx || j < 0 || j >= a.ny || k < 0 || k >= a.nz) {
     if (a.bc == GB_BC_DIRICHLET) return E::outside(a.out_re, a.out_im);
     // Neumann/periodic remap all three indices like the reference does
@@ -271,9 +270,9 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_bands(bool lap, typename Elem
 constexpr int kFdTY = 8, kFdTZ = 32, kFdXC = 16;
 static_assert(kFdTY * kFdTZ == kFdThreads, "one thread per tile column");
 
-template <typename T, bool REAL> struct FdTile {
-  using E = Elem<T, REAL>;
-  using V = typename E::V;
+template <typename T> struct FdTile {
+  using E = Elem<T, false>;
+  using V = C2<T>;
   V xm, c, xp, xq;  // this thread's column, planes i-1, i, i+1, i+2
   V h, hn;          // its halo point (if it owns one), planes i and i+1
   long hj, hk;      // halo point (y, z); may lie outside the grid
@@ -296,19 +295,19 @@ template <typename T, bool REAL> struct FdTile {
     // every thread of the tile loads its column, also past the far edge of
     // the grid (a partial tile): there fetch returns the boundary value the
     // last row/column needs as its neighbour
-    xm = fetch<T, REAL>(src, i0 - 1, j, k, a);
-    c = fetch<T, REAL>(src, i0, j, k, a);
-    xp = fetch<T, REAL>(src, i0 + 1, j, k, a);
+    xm = fetch<T>(src, i0 - 1, j, k, a);
+    c = fetch<T>(src, i0, j, k, a);
+    xp = fetch<T>(src, i0 + 1, j, k, a);
     xq = E::zero();
-    h = has_h ? fetch<T, REAL>(src, i0, hj, hk, a) : E::zero();
-    hn = has_h ? fetch<T, REAL>(src, i0 + 1, hj, hk, a) : E::zero();
+    h = has_h ? fetch<T>(src, i0, hj, hk, a) : E::zero();
+    hn = has_h ? fetch<T>(src, i0 + 1, hj, hk, a) : E::zero();
   }
 
   // loads of plane i + 2 (column and halo), issued at the top of step i;
   // returns the halo value for the shift
   __device__ __forceinline__ V prefetch(const V *src, const FdArgs &a, long i, long i1, long j, long k) {
-    if (i + 2 <= i1) xq = fetch<T, REAL>(src, i + 2, j, k, a);
-    return (has_h && i + 2 < i1) ? fetch<T, REAL>(src, i + 2, hj, hk, a) : E::zero();
+    if (i + 2 <= i1) xq = fetch<T>(src, i + 2, j, k, a);
+    return (has_h && i + 2 < i1) ? fetch<T>(src, i + 2, hj, hk, a) : E::zero();
   }
 
   __device__ __forceinline__ void shift(V hq) {
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic(const C2<T> *__restri
   const long i0 = blockIdx.z * (long) kFdXC;
   const long i1 = i0 + kFdXC < a.nx ? i0 + kFdXC : a.nx;
   const bool in = k < a.nz && j < a.ny;
-  FdTile<T, false> t;
+  FdTile<T> t;
   t.init(src, a, i0, j, k, ty, tz);
   double sx = 0.0, sy = 0.0;
   for (long i = i0; i < i1; i++) {
@@ -388,12 +387,14 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic(const C2<T> *__restri
   fd_block_sum(sx, sy, partial + ((long) blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
 }
 
-// The same sum with direct neighbour reads, for grids that L2 holds: CTAs walk
-// the chunks with a stride of the launch.  Energy call, tiles / direct: 100 / 78
-// us at 200 x 150 x 101 (48 MB of psi); 259 / 271 us at 256^3 (268 MB), where
-// L2 no longer holds what is read again.
-constexpr int kFdKinBlocks = 148 * 6;
-constexpr long kFdKinDirectBytes = 64L << 20;
+// The same sum with direct neighbour reads: CTAs walk the chunks with a stride of
+// the launch, faster until L2 no longer holds what is read again.  One sum, tiles
+// / direct, us: FP64 150^3 (54 MB of psi) 63 / 47, 180 x 181 x 183 (95 MB) 84 /
+// 71, 200^3 (128 MB) 95 / 87, 230 x 231 x 229 (195 MB) 129 / 118, 256^3 (268 MB)
+// 154 / 170; FP32, where the arithmetic is a larger part, 200^3 (64 MB) 91 / 80,
+// 205 x 205 x 203 (68 MB) 93 / 91, 220^3 (85 MB) 106 / 116.
+constexpr int kFdKinPerSm = 6;
+constexpr long fd_kin_direct_bytes(int prec) { return prec == GB_FP32 ? 64L << 20 : 192L << 20; }
 
 template <typename T>
 __global__ void __launch_bounds__(kFdThreads) k_fd_kinetic_direct(const C2<T> *__restrict__ src, FdArgs a,
@@ -458,7 +459,8 @@ __global__ void __launch_bounds__(256) k_finish_fd(const double2 *__restrict__ p
   }
 }
 
-// Launch grid of the tiled stencils: (z tiles, y tiles, x chunks).
+// Launch grid of the tiled kinetic sum: (z tiles, y tiles, x chunks).  Extents
+// beyond it are refused by the stencils too: one limit for all calls.
 int fd_grid(const gb_geom *g, dim3 *grid) {
   const long gz = (g->nz + kFdTZ - 1) / kFdTZ, gy = (g->ny + kFdTY - 1) / kFdTY, gx = (g->nx + kFdXC - 1) / kFdXC;
   if (gy > 65535 || gx > 65535) return gb__set_error(1005, "fd: grid too large for the stencil tiling");
@@ -551,8 +553,8 @@ extern "C" int gb_fd_kinetic_sum(const void *psi, const gb_geom *g, int bc, doub
   dim3 grid;
   if (fd_grid(g, &grid)) return gb_last_error();
   const long n = g->nx * g->ny * g->nz, chunks = (n + 2 * kFdThreads - 1) / (2 * kFdThreads);
-  const bool direct = n * (g->prec == GB_FP32 ? 8 : 16) <= kFdKinDirectBytes;
-  const long nb = !direct ? (long) grid.x * grid.y * grid.z : chunks < kFdKinBlocks ? chunks : kFdKinBlocks;
+  const bool direct = n * (g->prec == GB_FP32 ? 8 : 16) <= fd_kin_direct_bytes(g->prec);
+  const long nb = direct ? std::min(chunks, (long) kFdKinPerSm * gb__num_sms()) : (long) grid.x * grid.y * grid.z;
   double2 *partial = (double2 *) gb__scratch(GB_SCR_PARTIAL, sizeof(double2) * (size_t) nb);
   double2 *res = (double2 *) gb__result_slot();
   if (!partial || !res) return gb_last_error();

@@ -64,12 +64,21 @@ def test_stencils(b200, shape, bc):
         b200.free(x)
 
 
+# below and above the sizes from which the sum goes over halo tiles (192 MB of
+# psi in FP64, 64 MB in FP32), no extent there a multiple of a tile's
+KINETIC = [((2, 3, 5), 0), ((9, 17, 31), 0), ((20, 16, 32), 0), ((64, 100, 101), 0), ((233, 235, 231), 0),
+           ((9, 17, 31), 1), ((205, 207, 201), 1)]
+
+
 @pytest.mark.parametrize("bc,boundary", [("dirichlet", 1), ("neumann", 2), ("periodic", 3)])
-@pytest.mark.parametrize("shape", [(2, 3, 5), (9, 17, 31), (20, 16, 32), (64, 100, 101)])
-def test_kinetic_energy(b200, shape, bc, boundary):
+@pytest.mark.parametrize("shape,fp32", KINETIC)
+def test_kinetic_energy(b200, shape, fp32, bc, boundary):
     rng, step, mass = np.random.default_rng(sum(shape)), 0.3, 1.5
     psi = rng.uniform(-1, 1, shape) + 1j * rng.uniform(-1, 1, shape)
     w = b200.wf(*shape, step, mass, boundary, capi.WF_2ND_ORDER_CN, values=psi)
+    if fp32:
+        w.precision(capi.GRID_PREC_FP32)
+        psi = psi.astype(np.complex64).astype(complex)  # what the sum reads
     want = (-0.5 / mass * np.vdot(psi, _laplace(psi, step, bc)) * step**3).real
     kinetic = b200.lib.grid_wf_kinetic_energy_cn
     kinetic.restype = C.c_double
