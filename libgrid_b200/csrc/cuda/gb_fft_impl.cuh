@@ -658,6 +658,7 @@ __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsig
   if (!s_last) return;
   __threadfence();
   double s = 0.0;
+#pragma unroll 8
   for (unsigned i = threadIdx.x; i < nblk; i += THREADS) s += ld_cg(a.partial + i);
   r = sum(s);
   if (threadIdx.x == 0) {
