@@ -25,7 +25,8 @@ inline int active_axes(const gb_geom *g, int *ax) {
   return na;
 }
 
-inline PassArgs base_args(const gb_geom *g) {
+// step: passes of a split-operator step (pass_overlaps)
+inline PassArgs base_args(const gb_geom *g, bool step) {
   PassArgs a;
   memset(&a, 0, sizeof(a));
   a.nx = g->nx;
@@ -33,6 +34,7 @@ inline PassArgs base_args(const gb_geom *g) {
   a.nz = g->nz;
   a.scale = 1.0;
   a.kscale = 1.0;
+  a.step = step;
   return a;
 }
 
@@ -158,7 +160,7 @@ template <typename T> int gb__fft3d_t(void *data, const gb_geom *g, int sign, do
     if (scale != 1.0) return gb_complex_op(GB_OP_SCALE, data, nullptr, nullptr, 1, scale, 0.0, g->prec);
     return 0;
   }
-  PassArgs a = base_args(g);
+  PassArgs a = base_args(g, false);
   a.scale = scale;
   for (int s = 0; s < na; s++) {
     const bool last = (s == na - 1);
@@ -178,7 +180,7 @@ int gb__split_step_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const g
   using namespace gbfft;
   int ax[3];
   const int na = active_axes(g, ax);
-  PassArgs a = base_args(g);
+  PassArgs a = base_args(g, true);
   GbKinTables kt;
   GB_TRY(gb__kin_tables(g, kin, 0, &kt));
   for (int d = 0; d < 3; d++) {
@@ -237,7 +239,7 @@ int gb__split_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const 
     for (int s = 0; s < nsteps; s++) GB_TRY(gb__split_step_t<T>(psi, g, kin, pot));
     return 0;
   }
-  PassArgs ah = base_args(g);
+  PassArgs ah = base_args(g, true);
   GbKinTables kt;
   GB_TRY(gb__kin_tables(g, kin, 0, &kt));
   for (int d = 0; d < 3; d++) {
@@ -308,7 +310,7 @@ int gb__relax_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const 
   const int na = active_axes(g, ax);
   if (nsteps <= 0) return 0;
   if (na < 2 || !pot) return gb__set_error(1008, "relaxation steps: two axes and a potential needed");
-  PassArgs a = base_args(g);
+  PassArgs a = base_args(g, true);
   GbKinTables kt;
   GB_TRY(gb__kin_tables(g, kin, 0, &kt));
   for (int d = 0; d < 3; d++) {
@@ -370,7 +372,7 @@ template <typename T> int gb__ksq_sum_t(const void *psi, void *work, const gb_ge
   kin.scale = 1.0;
   GbKinTables kt;
   GB_TRY(gb__kin_tables(g, &kin, 1, &kt));
-  PassArgs a = base_args(g);
+  PassArgs a = base_args(g, false);
   for (int d = 0; d < 3; d++) {
     a.kfac[d] = kt.kfac[d];
     a.ksq[d] = kt.ksq[d];

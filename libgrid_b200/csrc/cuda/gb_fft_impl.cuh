@@ -275,6 +275,7 @@ struct PassArgs {
   double ntarget, nfactor;
   const double *pscale;
   int nlast;
+  int step;             // a pass of a split-operator step
   int *errflag;         // pipelined passes: set when a bounded wait gives up
 };
 
@@ -677,20 +678,23 @@ __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsig
 // blocks of 8) 440 / 280; 16 x 512 x 512 (32768) 4760 / 1850.
 inline bool norm_in_pass(long nblk) { return nblk <= 256; }
 
-// Whether the line passes over a grid overlap (gb_common.cuh).  Small grids
-// are bound by what lies between two kernels.  A large one comes from HBM, and
-// the CTAs that have waited all start their loads at once and stay in step:
-// loads, transforms and stores no longer overlap each other.  One step, launch
-// by launch / overlapped, us.  FP64: 32^3 39.1 / 21.6; 64^3 45.4 / 33.4;
-// 128^3 (34 MB) 138 / 126; 67 MB: 512 x 128 x 64 243 / 222, 256 x 128 x 128
-// 248 / 245, 512 x 64 x 128 261 / 265, 1 x 2048 x 2048 294 / 298; 134 MB:
-// 32 x 512 x 512 560 / 652, 512 x 128 x 128 554 / 664, 1024 x 128 x 64 563 /
-// 547; 268 MB: 64 x 512 x 512 1060 / 1267.  FP32, whose transforms take less:
-// 134 MB: 512 x 128 x 256 592 / 582, 256^3 475 / 467; 268 MB, five steps:
-// 512 x 256 x 256 3045 / 3134, 128 x 512 x 512 3327 / 3359.  A pipelined pass,
-// one wave of persistent CTAs that load ahead, always overlaps.
-template <typename T> bool pass_overlaps(const PassArgs &a) {
-  return (size_t) (a.nx * a.ny * a.nz) * sizeof(C2<T>) <= (sizeof(T) == 8 ? 64ul << 20 : 128ul << 20);
+// Whether the line passes over a grid overlap (gb_common.cuh).  Small grids are
+// bound by what lies between two kernels.  The passes of a step over a large one,
+// which comes from HBM, are slower when they overlap: CTAs that have waited start
+// their loads at once and stay in step, and loads, transforms and stores no longer
+// overlap each other.  One step, launch by launch / overlapped, us.  FP64: 32^3
+// 39.1 / 21.6; 64^3 45.4 / 33.4; 128^3 (34 MB) 138 / 126; 67 MB: 512 x 128 x 64
+// 243 / 222, 256 x 128 x 128 248 / 245, 512 x 64 x 128 261 / 265, 1 x 2048 x 2048
+// 294 / 298; 134 MB: 32 x 512 x 512 560 / 652, 512 x 128 x 128 554 / 664, 1024 x
+// 128 x 64 563 / 547; 268 MB: 64 x 512 x 512 1060 / 1267.  FP32, whose transforms
+// take less: 134 MB: 512 x 128 x 256 592 / 582, 256^3 475 / 467; 268 MB, five
+// steps: 512 x 256 x 256 3045 / 3134, 128 x 512 x 512 3327 / 3359.  Plain
+// transforms, one operation a pass, gain at every size where the lines are of up
+// to 512 points: forward and back, FP64, 512 x 256 x 64 (134 MB) 274 / 260, 256^3
+// 509 / 494, 64 x 512 x 512 537 / 525.
+// A pipelined pass, one wave of persistent CTAs that load ahead, always overlaps.
+template <typename T, int N> bool pass_overlaps(const PassArgs &a) {
+  return (!a.step && N <= 512) || (size_t) (a.nx * a.ny * a.nz) * sizeof(C2<T>) <= (sizeof(T) == 8 ? 64ul << 20 : 128ul << 20);
 }
 
 // ---------------------------------------------------------------- kernels
@@ -980,7 +984,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       const long nb = (outer + Cfg::L - 1) / Cfg::L;
       if (nblocks) *nblocks = nb;
-      launch_stream(pass_overlaps<T>(a), kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst,
+      launch_stream(pass_overlaps<T, N>(a), kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst,
                     outer, a);
     }
   } else {
@@ -1001,7 +1005,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) (inner / BZ), (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      bool overlap = pass_overlaps<T>(a);
+      bool overlap = pass_overlaps<T, N>(a);
       if constexpr (THREADS < 32) {
         if (!overlap || (long) grid.x * grid.y > kTinyOverlap<N>) {
           overlap = false;
@@ -1021,7 +1025,7 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       }
       dim3 grid((unsigned) inner, (unsigned) outer);
       if (nblocks) *nblocks = (long) grid.x * grid.y;
-      launch_stream(pass_overlaps<T>(a), kern, grid, N / Sched<N>::P, sm, st, (const T2 *) src, (T2 *) dst, inner,
+      launch_stream(pass_overlaps<T, N>(a), kern, grid, N / Sched<N>::P, sm, st, (const T2 *) src, (T2 *) dst, inner,
                     norm_args(a, grid, OpL<Ops...>{}));
       if constexpr (has_norm(OpL<Ops...>{})) return norm_after(a, grid);
     } else {

@@ -29,5 +29,7 @@ def test_no_cache_hint_intrinsics(name):
 
 def test_tables_built_on_the_stream_are_read_after_a_plain_launch():
     """Every sweep's launch takes the word of the function that builds tables."""
-    launches = re.findall(r"cn_launch\((.*?)\);", _code("gb_cn.cu").split("int gb_cn_step")[1])
-    assert launches and all(a.split(",")[-1].strip() == "built" for a in launches)
+    code = _code("gb_cn.cu")
+    launches = re.findall(r"cn_launch\w*(?:<\w+>)?\((.*?)\)+;", code.split("int gb_cn_step")[1])
+    assert len(launches) == 2 and all(a.split(",")[-1].strip() == "built" for a in launches)
+    assert "overlap = !built &&" in code
