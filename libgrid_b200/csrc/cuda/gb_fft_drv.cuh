@@ -349,7 +349,11 @@ int gb__relax_steps_t(void *psi, const gb_geom *g, const gb_kinetic *kin, const 
       GB_TRY(plane_mid<T>(g, psi, ap, true));
     } else {
       for (int s = na - 2; s >= 1; s--) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_INV>{})));
-      GB_TRY(line_pot_pass<T>(g, ax[0], psi, ap));
+      // in imaginary time the program for every potential is the faster one on
+      // short lines (128^3 FP64 22.9 us a pass against 24.4, 1 x 2048 x 2048 75.4
+      // against 66.6)
+      if (ax[0] == 2 && g->nz <= 256) GB_TRY((pass<T>(g, ax[0], psi, psi, ap, OpL<OP_INV, OP_POT, OP_FWD>{})));
+      else GB_TRY(line_pot_pass<T>(g, ax[0], psi, ap));
       for (int s = 1; s < na - 1; s++) GB_TRY((pass<T>(g, ax[s], psi, psi, a, OpL<OP_FWD>{})));
     }
   }

@@ -694,7 +694,8 @@ inline bool norm_in_pass(long nblk) { return nblk <= 256; }
 // 509 / 494, 64 x 512 x 512 537 / 525.
 // A pipelined pass, one wave of persistent CTAs that load ahead, always overlaps.
 template <typename T, int N> bool pass_overlaps(const PassArgs &a) {
-  return (!a.step && N <= 512) || (size_t) (a.nx * a.ny * a.nz) * sizeof(C2<T>) <= (sizeof(T) == 8 ? 64ul << 20 : 128ul << 20);
+  const size_t bytes = (size_t) (a.nx * a.ny * a.nz) * sizeof(C2<T>);
+  return (!a.step && N <= 512) || bytes <= (sizeof(T) == 8 ? 64ul << 20 : 128ul << 20);
 }
 
 // ---------------------------------------------------------------- kernels
@@ -963,6 +964,11 @@ inline int norm_after(const PassArgs &a, dim3 grid) {
 // 256 (8192) 108.6, 111.6.
 template <int N> constexpr long kTinyOverlap = N < 16 ? 4096 : 8192;
 
+// Programs that only contiguous lines of up to 256 points take (the relaxation
+// steps).
+template <int... Ops> struct ShortOnly { static constexpr bool value = false; };
+template <> struct ShortOnly<OP_INV, OP_POT, OP_FWD> { static constexpr bool value = true; };
+
 // Launch one pass of program Ops along `axis` for line length N.
 template <typename T, int N, int... Ops>
 int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, long inner, long *nblocks) {
@@ -970,7 +976,9 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
   // per-thread staging of the potential values (P reals per thread)
   constexpr size_t STAGE = has_stage(OpL<Ops...>{}) ? (size_t) Sched<N>::P * sizeof(T) : 0;
   cudaStream_t st = gb__stream();
-  if (inner == 1) {
+  if constexpr (ShortOnly<Ops...>::value && N > 256) {
+    return gb__set_error(1007, "fft pass: a program of short lines");
+  } else if (inner == 1) {
     if constexpr (has_norm(OpL<Ops...>{})) {  // the outermost of two or more axes is never contiguous
       return gb__set_error(1007, "fft pass: contiguous renormalising pass");
     } else {
@@ -987,6 +995,8 @@ int launch_pass_n(const void *src, void *dst, const PassArgs &a, long outer, lon
       launch_stream(pass_overlaps<T, N>(a), kern, dim3((unsigned) nb), Cfg::THREADS, sm, st, (const T2 *) src, (T2 *) dst,
                     outer, a);
     }
+  } else if constexpr (ShortOnly<Ops...>::value) {
+    return gb__set_error(1007, "fft pass: a program of contiguous lines");
   } else {
     constexpr int BZ = StridedCfg<N, sizeof(T)>::BZ;
     if (!nblocks) {
