@@ -158,9 +158,11 @@ __device__ __forceinline__ double2 cn_rhs(long i, long n, int bc, double2 cp, do
 // Potential factor on the elements i = i0, i0 + di, ... < n of one tile line
 // or column whose element i sits at base[i * es]; V of element i at
 // vbase + i * vstep, coordinates (ix, iy, iz) with the line's own axis
-// running along i.  No division per element; V loads batched by B.
-__device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int di, int n, long vbase, long vstep,
-                                             long ix, long iy, long iz, const CnAxis &a, const gb_potential &pt) {
+// running along i; vals: pt.v below the wait.  No division per element; V loads
+// batched by B.
+__device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int di, int n, const void *vals, long vbase,
+                                             long vstep, long ix, long iy, long iz, const CnAxis &a,
+                                             const gb_potential &pt) {
   constexpr int B = 4;
   for (int ib = i0; ib < n; ib += di * B) {
     double2 v[B];
@@ -173,8 +175,8 @@ __device__ __forceinline__ void cn_pot_elems(double2 *base, int es, int i0, int 
         // streaming loads: V is read once per sweep, and evict-first keeps
         // the solver's coefficient tables in the small L1 left beside the
         // shared-memory tiles
-        if (pt.kind == GB_POT_COMPLEX) v[k] = ld_cs((const double2 *) pt.v + vi);
-        else if (pt.kind == GB_POT_REAL) v[k].x = ld_cs((const double *) pt.v + vi);
+        if (pt.kind == GB_POT_COMPLEX) v[k] = ld_cs((const double2 *) vals + vi);
+        else if (pt.kind == GB_POT_REAL) v[k].x = ld_cs((const double *) vals + vi);
       }
     }
 #pragma unroll
@@ -199,6 +201,7 @@ __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, in
                                             const CnAxis &a, const gb_potential &pt) {
   const int n = (int) a.n, nthr = (int) blockDim.x;
   const long vrow = pt.vrow;
+  const void *vals = below_wait(pt.v);
   if constexpr (CONTIG) {
     for (int l = (int) (threadIdx.x >> 5); l < nl; l += nthr >> 5) {
       const long lid = line0 + l;
@@ -213,8 +216,8 @@ __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, in
         if (a.axis == 1) ix = lid;
         vstep = vrow;
       }
-      cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, (ix * a.ny + iy) * vrow, vstep, ix, iy, 0,
-                   a, pt);
+      cn_pot_elems(sm + (long) l * pitch, 1, (int) (threadIdx.x & 31), 32, n, vals, (ix * a.ny + iy) * vrow, vstep, ix,
+                   iy, 0, a, pt);
     }
   } else {
     const int l = (int) threadIdx.x % cols;
@@ -232,7 +235,7 @@ __device__ __forceinline__ void cn_tile_pot(double2 *sm, int pitch, int cols, in
       vbase = ix * a.ny * vrow + iz;
       vstep = vrow;
     }
-    cn_pot_elems(sm + l, pitch, (int) threadIdx.x / cols, nthr / cols, n, vbase, vstep, ix, iy, iz, a, pt);
+    cn_pot_elems(sm + l, pitch, (int) threadIdx.x / cols, nthr / cols, n, vals, vbase, vstep, ix, iy, iz, a, pt);
   }
 }
 

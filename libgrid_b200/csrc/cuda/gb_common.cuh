@@ -185,8 +185,9 @@ extern "C" cudaStream_t gb__stream(void);
 // - what a restrict pointer reads (as read-only loads) goes through the pointer
 //   that grid_wait was given;
 // - plain loads of other pointers, cp.async and bulk copies stay below it;
-// - the cache-hint intrinsics (__ldcg, __ldcs) are not known to: ld_cg and
-//   ld_cs take their place;
+// - the cache-hint intrinsics (__ldcg, __ldcs) are not known to: ld_cg (volatile)
+//   and ld_cs, through a pointer taken below the wait (below_wait), take their
+//   place;
 // - __ldg is for what no kernel can still be writing: tables are written by a
 //   kernel whose next one on the stream was launched without overlap.
 // Which launches overlap: pass_overlaps in gb_fft_impl.cuh, cn_launch in
@@ -202,14 +203,21 @@ __device__ __forceinline__ double ld_cg(const double *p) {
   asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
+// The pointer, known to the compiler only from here on.
+template <typename P> __device__ __forceinline__ P below_wait(P p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+// Streaming loads of what no one writes after the wait; free to be scheduled
+// between it and their use.
 __device__ __forceinline__ double ld_cs(const double *p) {
   double v;
-  asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ double2 ld_cs(const double2 *p) {
   double2 v;
-  asm volatile("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  asm("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
 }
 

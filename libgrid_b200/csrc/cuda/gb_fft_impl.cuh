@@ -659,8 +659,13 @@ __device__ __forceinline__ void norm_finish(double acc, const PassArgs &a, unsig
   if (!s_last) return;
   __threadfence();
   double s = 0.0;
-#pragma unroll 8
-  for (unsigned i = threadIdx.x; i < nblk; i += THREADS) s += ld_cg(a.partial + i);
+  for (unsigned i = threadIdx.x; i < nblk; i += 8 * THREADS) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = i + u * THREADS < nblk ? ld_cg(a.partial + i + u * THREADS) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) s += v[u];
+  }
   r = sum(s);
   if (threadIdx.x == 0) {
     const double nrm = r * a.nfactor;
